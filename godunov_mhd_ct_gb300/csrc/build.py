@@ -30,7 +30,7 @@ UNITS = {
     "amr.cu": ["--fmad=false"],
     "forest.cpp": ["-Xcompiler", "-pthread"],
 }
-HEADERS = ["mhd_math.cuh", "fused_step.cuh", "column_step.cuh", "launch.cuh",
+HEADERS = ["mhd_math.cuh", "fused_step.cuh", "column_step.cuh", "launch.cuh", "cfl_screen.cuh",
            os.path.join("..", "..", "include", "gmhd.h")]
 
 

@@ -22,6 +22,7 @@
 #include <mutex>
 
 #include "../../include/gmhd.h"
+#include "cfl_screen.cuh"
 #include "mhd_math.cuh"
 
 namespace
@@ -65,16 +66,16 @@ clear_slots_kernel(unsigned long long * slots, int n)
     slots[kFlagSlot] = 0ull;
 }
 
-// compute_cfl (scheme/ComputeDtMHDFunctor.cpp:86-151) per owned cell, one CTA per block, max per
-// problem into slots[]. All blocks at one level (cell size dx). A block whose problem id is not in
-// [0, np) does no work and sets the flag slot.
+// compute_cfl (scheme/ComputeDtMHDFunctor.cpp:86-151) per owned cell, `chunks` CTAs per block, max per
+// problem into slots[], screened in FP32 (cfl_screen.cuh). All blocks at one level (cell size dx, 1/dx in FP32
+// in idx). A block whose problem id is not in [0, np) does no work and sets the flag slot.
 __global__ void __launch_bounds__(256)
 inv_dt_noalloc_kernel(const double * __restrict__ U, const double * __restrict__ B,
-                      const int32_t * __restrict__ problem, int np, int dim, int bx, int by, int bz, int64_t ncell,
-                      int64_t nfx, int64_t nfy, int64_t nface, double dx, double gamma0, double smallr,
-                      double smallp, Sources src, unsigned long long * slots)
+                      const int32_t * __restrict__ problem, int np, int chunks, int dim, int bx, int by, int64_t ncell,
+                      int64_t nfx, int64_t nfy, int64_t nface, double dx, float idx, double gamma0, float gm1,
+                      double smallr, double smallp, Sources src, unsigned long long * slots)
 {
-  const int blk = blockIdx.x;
+  const int blk = blockIdx.x / chunks, chunk = blockIdx.x - blk * chunks;
   const int pid = problem ? problem[blk] : 0;
   if ((unsigned)pid >= (unsigned)np)
   {
@@ -83,29 +84,9 @@ inv_dt_noalloc_kernel(const double * __restrict__ U, const double * __restrict__
       atomicExch(&slots[kFlagSlot], 1ull);
     return;
   }
-  const double *Ub = U + (int64_t)blk * 5 * ncell;
-  const double *Bb = B + (int64_t)blk * nface;
-  double        m = 0.0;
-  for (int64_t c = threadIdx.x; c < ncell; c += blockDim.x)
-  {
-    const int i = (int)(c % bx), j = (int)((c / bx) % by), k = (int)(c / ((int64_t)bx * by));
-    m = fmax(m, gmhd::cell_inv_dt_fp64(Ub, Bb, dim, bx, by, i, j, k, c, ncell, nfx, nfy, dx, gamma0, smallr, smallp,
-                                       src));
-  }
-  __shared__ double red[8];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
-  if ((threadIdx.x & 31) == 0)
-    red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0)
-  {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-      m = fmax(m, red[w]);
-    // positive doubles order like their bit patterns
-    atomicMax(&slots[pid], (unsigned long long)__double_as_longlong(m));
-  }
+  gmhd::screened_inv_dt(U + (int64_t)blk * 5 * ncell, B + (int64_t)blk * nface, dim, bx, by,
+                        (int64_t)chunk * 256 * gmhd::kScreenCells, ncell, nfx, nfy, idx, gamma0, gm1, smallr, smallp, src,
+                        [&]() { return dx; }, &slots[pid]);
 }
 
 // Per-problem results, or NaN everywhere when some block had a problem id out of range.
@@ -162,10 +143,16 @@ gmhd_inv_dt_noalloc(const gmhd_params * params, int32_t dim, int32_t bx, int32_t
   // an error left by earlier, unrelated work is not this call's: clear it so that the check after the
   // launches reports only these
   (void)cudaGetLastError();
+  const int64_t chunks = (ncell + 256 * gmhd::kScreenCells - 1) / (256 * gmhd::kScreenCells);
+  if (ncell > 0xffffffffLL || (int64_t)n_blocks * chunks > 0x7fffffffLL)
+    return GMHD_ERR_CUDA;
   clear_slots_kernel<<<(np + 255) / 256, 256, 0, s>>>(slots, np);
   if (n_blocks > 0)
-    inv_dt_noalloc_kernel<<<n_blocks, 256, 0, s>>>(U, B, problem, np, dim, bx, by, bz, ncell, nfx, nfy, nface, dx,
-                                                   params->gamma0, params->smallr, smallp, src, slots);
+    inv_dt_noalloc_kernel<<<(unsigned)(n_blocks * chunks), 256, 0, s>>>(U, B, problem, np, (int)chunks, dim, bx, by,
+                                                                        ncell, nfx, nfy, nface, dx, (float)(1.0 / dx),
+                                                                        params->gamma0, (float)(params->gamma0 - 1.0),
+                                                                        params->smallr, smallp, src,
+                                                                        slots);
   write_out_kernel<<<(np + 255) / 256, 256, 0, s>>>(slots, inv_dt, np);
   return cudaGetLastError() == cudaSuccess ? GMHD_OK : GMHD_ERR_CUDA;
 }

@@ -2,6 +2,7 @@
 // --fmad=false so that every a*b+c stays unfused, matching the reference formulas' FP64 rounding.
 #include <type_traits>
 
+#include "cfl_screen.cuh"
 #include "launch.cuh"
 
 namespace gmhd
@@ -100,37 +101,22 @@ prepare_fp64()
 
 namespace gmhd
 {
-// ComputeDtMHDFunctor::compute_cfl (scheme/ComputeDtMHDFunctor.cpp:86-151) over the owned blocks,
-// one CTA per block, max-reduced per problem. FP64 with the reference operand order.
+// ComputeDtMHDFunctor::compute_cfl (scheme/ComputeDtMHDFunctor.cpp:86-151) over the owned blocks, max-reduced
+// per problem: FP64 with the reference operand order where the FP32 screen (cfl_screen.cuh) leaves a cell in
+// question. A CTA takes 1024 cells of one block, so that a mesh of few large blocks fills the device too: one
+// CTA per 32^3 block left 152 SMs with 3.4 CTAs each.
 __global__ void __launch_bounds__(256)
 inv_dt_kernel(const double * __restrict__ U, const double * __restrict__ B, const int32_t * __restrict__ level,
-              const int32_t * __restrict__ problem, int dim, int bx, int by, int bz, int64_t ncell, int64_t nfx,
-              int64_t nfy, int64_t nface, double gamma0, double smallr, double smallp, double scaling_factor,
-              Sources src, unsigned long long * invdt)
+              const int32_t * __restrict__ problem, int chunks, int dim, int bx, int by, int64_t ncell, int64_t nfx,
+              int64_t nfy, int64_t nface, double gamma0, float gm1, double smallr, double smallp,
+              double scaling_factor, float inv_scaling, Sources src, unsigned long long * invdt)
 {
-  const int     blk = blockIdx.x;
-  const double  dx = (1.0 / (double)((int64_t)bx << level[blk])) * scaling_factor;
-  const double *Ub = U + (int64_t)blk * 5 * ncell;
-  const double *Bb = B + (int64_t)blk * nface;
-  double        m = 0.0;
-  for (int64_t c = threadIdx.x; c < ncell; c += blockDim.x)
-  {
-    const int i = (int)(c % bx), j = (int)((c / bx) % by), k = (int)(c / ((int64_t)bx * by));
-    m = fmax(m, cell_inv_dt_fp64(Ub, Bb, dim, bx, by, i, j, k, c, ncell, nfx, nfy, dx, gamma0, smallr, smallp, src));
-  }
-  __shared__ double red[8];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
-  if ((threadIdx.x & 31) == 0)
-    red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0)
-  {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-      m = fmax(m, red[w]);
-    atomicMax(&invdt[problem ? problem[blk] : 0], (unsigned long long)__double_as_longlong(m));
-  }
+  const int     blk = blockIdx.x / chunks, chunk = blockIdx.x - blk * chunks;
+  const int64_t cells = (int64_t)bx << level[blk];
+  auto          dx_of = [&]() { return (1.0 / (double)cells) * scaling_factor; };
+  screened_inv_dt(U + (int64_t)blk * 5 * ncell, B + (int64_t)blk * nface, dim, bx, by,
+                  (int64_t)chunk * 256 * kScreenCells, ncell, nfx, nfy, (float)cells * inv_scaling, gamma0, gm1, smallr,
+                  smallp, src, dx_of, &invdt[problem ? problem[blk] : 0]);
 }
 
 int
@@ -141,8 +127,13 @@ launch_inv_dt(const double * U, const double * B, const int32_t * level, const i
 {
   if (n_owned <= 0)
     return 0;
-  inv_dt_kernel<<<n_owned, 256, 0, stream>>>(U, B, level, problem, dim, bx, by, bz, ncell, nfx, nfy, nface, gamma0,
-                                             smallr, smallp, scaling_factor, src, invdt);
+  (void)bz;
+  const int64_t chunks = (ncell + 256 * kScreenCells - 1) / (256 * kScreenCells);
+  if (ncell > 0xffffffffLL || (int64_t)n_owned * chunks > 0x7fffffffLL)
+    return (int)cudaErrorInvalidConfiguration;
+  inv_dt_kernel<<<(unsigned)(n_owned * chunks), 256, 0, stream>>>(U, B, level, problem, (int)chunks, dim, bx, by, ncell,
+                                                                  nfx, nfy, nface, gamma0, (float)(gamma0 - 1.0), smallr,
+                                                                  smallp, scaling_factor, (float)(1.0 / scaling_factor), src, invdt);
   return (int)cudaGetLastError();
 }
 } // namespace gmhd

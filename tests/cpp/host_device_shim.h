@@ -1,0 +1,86 @@
+// Lets the device math headers compile as host C++ for the CPU checks: CUDA's qualifiers and the few intrinsics
+// those headers use.
+#pragma once
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#define __device__
+#define __host__
+#define __forceinline__ inline
+#define __restrict__
+
+static inline long long
+__double_as_longlong(double x)
+{
+  long long r;
+  std::memcpy(&r, &x, 8);
+  return r;
+}
+static inline double
+__longlong_as_double(long long x)
+{
+  double r;
+  std::memcpy(&r, &x, 8);
+  return r;
+}
+static inline int
+__float_as_int(float x)
+{
+  int r;
+  std::memcpy(&r, &x, 4);
+  return r;
+}
+static inline unsigned
+__float_as_uint(float x)
+{
+  return (unsigned)__float_as_int(x);
+}
+static inline float
+__uint_as_float(unsigned x)
+{
+  float r;
+  std::memcpy(&r, &x, 4);
+  return r;
+}
+static inline float
+__int_as_float(int x)
+{
+  return __uint_as_float((unsigned)x);
+}
+static inline int
+__double2hiint(double x)
+{
+  return (int)(__double_as_longlong(x) >> 32);
+}
+static inline int
+__double2loint(double x)
+{
+  return (int)(uint32_t)__double_as_longlong(x);
+}
+static inline double
+__hiloint2double(int hi, int lo)
+{
+  return __longlong_as_double((long long)(((uint64_t)(uint32_t)hi << 32) | (uint32_t)lo));
+}
+static inline unsigned
+__funnelshift_l(unsigned lo, unsigned hi, unsigned s)
+{
+  return (unsigned)(((((uint64_t)hi << 32) | lo) << (s & 31)) >> 32);
+}
+static inline uint64_t
+__umul64hi(uint64_t a, uint64_t b)
+{
+  return (uint64_t)(((unsigned __int128)a * b) >> 64);
+}
+static inline unsigned
+__umulhi(unsigned a, unsigned b)
+{
+  return (unsigned)(((uint64_t)a * b) >> 32);
+}
+static inline float
+rsqrtf(float x)
+{
+  return 1.0f / sqrtf(x);
+}
