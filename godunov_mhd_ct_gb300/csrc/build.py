@@ -31,6 +31,7 @@ UNITS = {
     "forest.cpp": ["-Xcompiler", "-pthread"],
 }
 HEADERS = ["mhd_math.cuh", "fused_step.cuh", "column_step.cuh", "launch.cuh", "cfl_screen.cuh",
+           "exact_solvers.cuh", "fp64_int.cuh",
            os.path.join("..", "..", "include", "gmhd.h")]
 
 

@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(K::NT, 2) column_step_kernel(const StepArgs a)
             {
               const int i = m % (TX + 1), j = m / (TX + 1);
               fg = (x0 + i) + (int64_t)(bx + 1) * ((y0 + j) + (int64_t)by * p);
-              const double d = curl2<false>(Mz[i + (TX + 1) * (j + 1)] - Mz[i + (TX + 1) * j],
+              const double d = curl2(Mz[i + (TX + 1) * (j + 1)] - Mz[i + (TX + 1) * j],
                                             My1[i + (TX + 1) * j] - My0[i + (TX + 1) * j]);
               bnew = Bblk[fg] + d;
               owned = i < TX || ex;
@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(K::NT, 2) column_step_kernel(const StepArgs a)
               const int i = n % TX, j = n / TX;
               fg = a.nfx + (x0 + i) + (int64_t)bx * ((y0 + j) + (int64_t)(by + 1) * p);
               const double d =
-                curl2<false>(Mx1[i + TX * j] - Mx0[i + TX * j], Mz[(i + 1) + (TX + 1) * j] - Mz[i + (TX + 1) * j]);
+                curl2(Mx1[i + TX * j] - Mx0[i + TX * j], Mz[(i + 1) + (TX + 1) * j] - Mz[i + (TX + 1) * j]);
               bnew = Bblk[fg] + d;
               owned = j < TY || ey;
               t.Ny()[n] = to_r<float>(bnew);
@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(K::NT, 2) column_step_kernel(const StepArgs a)
               const int i = n % TX, j = n / TX;
               const double * MxL = t.Mx(L), *MyL = t.My(L);
               fg = a.nfx + a.nfy + (x0 + i) + (int64_t)bx * ((y0 + j) + (int64_t)by * L);
-              const double d = curl2<false>(MyL[(i + 1) + (TX + 1) * j] - MyL[i + (TX + 1) * j],
+              const double d = curl2(MyL[(i + 1) + (TX + 1) * j] - MyL[i + (TX + 1) * j],
                                             MxL[i + TX * (j + 1)] - MxL[i + TX * j]);
               bnew = Bblk[fg] + d;
               owned = true;

@@ -36,6 +36,7 @@ struct StepArgs
   int     tiles_x, tiles_y, tiles_z;
   int64_t ncell, nfx, nfy, nface;
   double  gamma0, smallr, smallc, smallp, slope_type, scaling_factor, cfl;
+  double  entho; // 1 / (gamma0 - 1)
   // the same in FP32 for the mixed path (converted once on the host: each FP64 conversion in the
   // kernel is an FP64-pipe instruction per warp)
   float   gamma0_f, smallr_f, smallc_f, smallp_f, slope_type_f;
@@ -223,16 +224,23 @@ viscous_face_flux(const typename C::R * vel, int dir, int i, int j, int k, typen
   R             v[3], g[3][3];
   const int     c0 = C::vi(i, j, k);
   const int     cx = C::vi(i - 1, j, k), cy = C::vi(i, j - 1, k), cz = C::D3 ? C::vi(i, j, k - 1) : c0;
+  const auto    idx = recip<R>(dx);
+  auto          by_dx = [&](R x) -> R {
+    if constexpr (C::EXACT)
+      return div64(x, idx);
+    else
+      return x / dx;
+  };
 #pragma unroll
   for (int c = 0; c < NC; ++c)
   {
     const R * V = vel + c * C::NVEL;
     const R   qr = V[c0];
     v[c] = qr;
-    g[c][0] = (qr - V[cx]) / dx;
-    g[c][1] = (qr - V[cy]) / dx;
+    g[c][0] = by_dx(qr - V[cx]);
+    g[c][1] = by_dx(qr - V[cy]);
     if constexpr (C::DIM == 3)
-      g[c][2] = (qr - V[cz]) / dx;
+      g[c][2] = by_dx(qr - V[cz]);
   }
   R fu, fv, fw = R(0), fe;
   if constexpr (C::DIM == 2)
@@ -320,7 +328,7 @@ fine_face_flux(const StepArgs & a, int blk, int slot, int d, int side, int g1, i
         acc += a.flux_side[(((int64_t)cs * 2 * C::DIM + ff) * C::NFS + var) * a.flux_face_stride + F1 +
                            (int64_t)bs[t1] * F2];
     }
-  return acc / (double)(1 << C::DIM);
+  return dscale_down(acc, C::DIM);
 }
 
 // Asynchronous global -> shared copies (cp.async, sm_80+): 8 bytes through L1, 16 bytes bypassing it.
@@ -409,6 +417,13 @@ f_index(int i, int j, int k)
   return CMP == 0 ? C::fxi(i, j, k) : (CMP == 1 ? C::fyi(i, j, k) : C::fzi(i, j, C::D3 ? k : 0));
 }
 
+// acc / count of 1 to 4 values
+__device__ __forceinline__ double
+mean_of(double acc, int count)
+{
+  return count == 3 ? div64(acc, 3.0) : (count == 1 ? acc : (count == 2 ? dscale_down(acc, 1) : div64(acc, (double)count)));
+}
+
 // CorrectEmfAtBlockBorderFunctor::correct_emf (CorrectEmfAtBlockBorderFunctor.cpp:94-360) of a
 // block-border edge on a coarse/fine mesh. Siblings are the regions across the two transverse block
 // borders (v0 along D0, v1 along D1) and across both. Same-level copies are this tile's own value
@@ -467,7 +482,7 @@ amr_border_emf(const TileView<C> & t, const int * gi, int v0, int v1, typename C
           acc += to_d<R>(val);
           ++count;
         }
-      out = acc / (double)count;
+      out = mean_of(acc, count);
     }
   }
   else if (finer)
@@ -507,7 +522,7 @@ amr_border_emf(const TileView<C> & t, const int * gi, int v0, int v1, typename C
         acc += E[e + (CD == 0 ? 1 : (CD == 1 ? (int64_t)sx : (int64_t)sx * sy))];
       ++count;
     }
-    out = acc / (double)count / (double)(1 << (C::DIM - 1));
+    out = dscale_down(mean_of(acc, count), C::DIM - 1);
   }
   if (all_same && C::EXACT)
   {
@@ -521,7 +536,7 @@ amr_border_emf(const TileView<C> & t, const int * gi, int v0, int v1, typename C
         acc += to_d<R>(val);
         ++count;
       }
-    out = acc / (double)count;
+    out = mean_of(acc, count);
   }
   return out;
 }
@@ -634,35 +649,36 @@ recon_edge(const TileView<C> & t, int sc, int fb0, int fb1, typename C::R * q)
   const R * S0 = t.sl + D0 * 8 * NS + sc;
   const R * S1 = t.sl + D1 * 8 * NS + sc;
   const R   g0 = (R)sd0, g1 = (R)sd1;
-  auto      h = [&](int v) { return R(0.5) * (g0 * S0[v * NS] + g1 * S1[v * NS]); };
+  auto      h = [&](int v) { q[v] = plus_half<R>(q[v], g0 * S0[v * NS] + g1 * S1[v * NS]); };
 #pragma unroll
   for (int v = 0; v < 5; ++v)
-    q[v] += h(v);
+    h(v);
+  const R E0 = plus_half<R>(B0, (R)sb0 * dB0d1), E1 = plus_half<R>(B1, (R)sb1 * dB1d0);
   if constexpr (C::DIM == 2)
   {
-    q[IA] = B0 + R(0.5) * ((R)sb0 * dB0d1);
-    q[IB] = B1 + R(0.5) * ((R)sb1 * dB1d0);
-    q[IC] += h(IC);
+    q[IA] = E0;
+    q[IB] = E1;
+    h(IC);
   }
   else
   {
     // the reference's branch order for IA / IB / IC (ComputeEmfAndStoreFunctor.cpp:324-363)
     if constexpr (D0 == 0)
-      q[IA] = B0 + R(0.5) * ((R)sb0 * dB0d1);
+      q[IA] = E0;
     else
-      q[IA] += h(IA);
+      h(IA);
     if constexpr (D0 == 1)
-      q[IB] = B0 + R(0.5) * ((R)sb0 * dB0d1);
-    else
-      q[IB] += h(IB);
+      q[IB] = E0;
+    else if constexpr (D1 != 1)
+      h(IB);
     if constexpr (D1 == 1)
-      q[IB] = B1 + R(0.5) * ((R)sb1 * dB1d0);
+      q[IB] = E1;
     else
-      q[IB] += h(IB);
+      h(IB);
     if constexpr (D1 == 2)
-      q[IC] = B1 + R(0.5) * ((R)sb1 * dB1d0);
+      q[IC] = E1;
     else
-      q[IC] += h(IC);
+      h(IC);
   }
   q[ID] = rmax<R>(t.ph.smallr, q[ID]);
   q[IP] = rmax<R>(t.ph.smallp * q[ID], q[IP]);
@@ -671,21 +687,11 @@ recon_edge(const TileView<C> & t, int sc, int fb0, int fb1, typename C::R * q)
 // EMFs along direction CD on the tile's edges [0, T] (ComputeEmfAndStoreFunctor.cpp:371-590), with
 // the border averaging of CorrectEmfAtBlockBorderFunctor (uniform level, .cpp:298-356)
 // Face increment of the CT update from two EMF differences: the reference's "d = 0; d += a; d -= b"
-// (ReadEmfAndUpdateFunctor.cpp:118-161) on the FP64 path; a - b on the mixed path, the same value
-// up to the sign of a zero, one FP64 instruction less per face.
-template <bool EXACT>
+// (ReadEmfAndUpdateFunctor.cpp:118-161) as a - b, the same value up to the sign of a zero.
 __device__ __forceinline__ double
 curl2(double a, double b)
 {
-  if constexpr (EXACT)
-  {
-    double d = 0;
-    d += a;
-    d -= b;
-    return d;
-  }
-  else
-    return a - b;
+  return a - b;
 }
 
 // Items of the phase-5 passes are dealt round-robin to the threads, each pass starting where the
@@ -711,76 +717,156 @@ face_count()
   return (C::TX + (D == 0)) * (C::TY + (D == 1)) * (C::TZ + (D == 2 && C::D3));
 }
 
+// The four reconstructed states around edge (i, j, k) along CD (item m of the direction's list)
+template <class C, int CD>
+__device__ __forceinline__ void
+edge_states(const TileView<C> & t, int i, int j, int k, typename C::R (*qe)[8])
+{
+  constexpr int D0 = CD == 0 ? 1 : 0;
+  constexpr int D1 = CD == 2 ? 1 : 2;
+  constexpr int s0 = s_stride<C>(D0), s1 = s_stride<C>(D1);
+  constexpr int f00 = f_stride<C>(D0, D0), f01 = f_stride<C>(D0, D1);
+  constexpr int f10 = f_stride<C>(D1, D0), f11 = f_stride<C>(D1, D1);
+  const int     sc = C::si(i, j, k);
+  const int     g0 = f_index<C, D0>(i, j, k);
+  const int     g1 = f_index<C, D1>(i, j, k);
+  recon_edge<C, D0, D1, LOC_LB>(t, sc, g0, g1, qe[ELB]);
+  recon_edge<C, D0, D1, LOC_RT>(t, sc - s0 - s1, g0 - f00 - f01, g1 - f10 - f11, qe[ERT]);
+  // y edges: the reference swaps the RB and LT states (ComputeEmfAndStoreFunctor.cpp:551-560)
+  recon_edge<C, D0, D1, LOC_RB>(t, sc - s0, g0 - f00, g1 - f10, qe[CD == 1 ? ELT : ERB]);
+  recon_edge<C, D0, D1, LOC_LT>(t, sc - s1, g0 - f01, g1 - f11, qe[CD == 1 ? ERB : ELT]);
+}
+
+// Stores the EMF val (times dt/dx) of edge (i, j, k) along CD, averaged with its sibling copies where four blocks
+// meet (self first, then the non-outside siblings); on a conforming mesh the copies are computed from identical data,
+// so the sum is of equal terms
+template <class C, int CD>
+__device__ __forceinline__ void
+store_emf(const TileView<C> & t, int i, int j, int k, typename C::R val)
+{
+  using R = typename C::R;
+  constexpr int D0 = CD == 0 ? 1 : 0;
+  constexpr int D1 = CD == 2 ? 1 : 2;
+  double        out;
+  const int gi[3] = {t.x0 + i, t.y0 + j, t.z0 + k};
+  const int bs[3] = {t.bx, t.by, t.bz};
+  const int v0 = gi[D0] == 0 ? -1 : (gi[D0] == bs[D0] ? 1 : 0);
+  const int v1 = (C::DIM == 2 && D1 == 2) ? 0 : (gi[D1] == 0 ? -1 : (gi[D1] == bs[D1] ? 1 : 0));
+  if constexpr (C::AMR)
+    out = amr_border_emf<C, CD, D0, D1>(t, gi, v0, v1, val);
+  else if (v0 != 0 && v1 != 0)
+  {
+    const int sl0 = nb_slot(D0 == 0 ? v0 : 0, D0 == 1 ? v0 : 0, 0);
+    const int sl1 = nb_slot(D1 == 0 ? v1 : 0, D1 == 1 ? v1 : 0, D1 == 2 ? v1 : 0);
+    const int sl2 = nb_slot(D0 == 0 ? v0 : (D1 == 0 ? v1 : 0), D0 == 1 ? v0 : (D1 == 1 ? v1 : 0), D1 == 2 ? v1 : 0);
+    const int n0 = t.s_nbr[sl0], n1 = t.s_nbr[sl1], n2 = t.s_nbr[sl2];
+    if (n0 >= 0 && n1 >= 0 && n2 >= 0)
+    {
+      R   acc = R(0);
+      int count = 1;
+      acc += val;
+      if (n0 < t.n_owned)
+      {
+        acc += val;
+        count++;
+      }
+      if (n1 < t.n_owned)
+      {
+        acc += val;
+        count++;
+      }
+      if (n2 < t.n_owned)
+      {
+        acc += val;
+        count++;
+      }
+      if constexpr (C::EXACT)
+        val = mean_of(acc, count);
+      else
+        val = acc / (R)count;
+    }
+  }
+  if constexpr (!C::AMR)
+    out = to_d<R>(val);
+  t.emfd[(C::DIM == 3 ? CD : 0) * C::NM + C::mi(i, j, k)] = out;
+}
+
 template <class C, int CD, int START>
 __device__ __forceinline__ void
 edge_pass(const TileView<C> & t, int tid)
 {
   using R = typename C::R;
-  constexpr int D0 = CD == 0 ? 1 : 0;
-  constexpr int D1 = CD == 2 ? 1 : 2;
   constexpr int NX = CD == 0 ? C::TX : C::TX + 1;
   constexpr int NY = CD == 1 ? C::TY : C::TY + 1;
   constexpr int NZ = C::DIM == 3 ? (CD == 2 ? C::TZ : C::TZ + 1) : 1;
-  constexpr int s0 = s_stride<C>(D0), s1 = s_stride<C>(D1);
-  constexpr int f00 = f_stride<C>(D0, D0), f01 = f_stride<C>(D0, D1);
-  constexpr int f10 = f_stride<C>(D1, D0), f11 = f_stride<C>(D1, D1);
   for (int m = first_item<C>(tid, START); m < NX * NY * NZ; m += C::NT)
   {
     const int i = m % NX, j = (m / NX) % NY, k = m / (NX * NY);
-    const int sc = C::si(i, j, k);
-    const int g0 = f_index<C, D0>(i, j, k);
-    const int g1 = f_index<C, D1>(i, j, k);
     R         qe[4][8];
-    recon_edge<C, D0, D1, LOC_LB>(t, sc, g0, g1, qe[ELB]);
-    recon_edge<C, D0, D1, LOC_RT>(t, sc - s0 - s1, g0 - f00 - f01, g1 - f10 - f11, qe[ERT]);
-    // y edges: the reference swaps the RB and LT states (ComputeEmfAndStoreFunctor.cpp:551-560)
-    recon_edge<C, D0, D1, LOC_RB>(t, sc - s0, g0 - f00, g1 - f10, qe[CD == 1 ? ELT : ERB]);
-    recon_edge<C, D0, D1, LOC_LT>(t, sc - s1, g0 - f01, g1 - f11, qe[CD == 1 ? ERB : ELT]);
-    R      val = edge_emf<R, CD>(qe, t.ph) * t.dtdx;
-    double out;
-    // an edge on a line where four blocks meet is averaged with its sibling copies (self first,
-    // then the non-outside siblings); on a conforming mesh the copies are computed from identical
-    // data, so the sum is of equal terms
-    {
-      const int gi[3] = {t.x0 + i, t.y0 + j, t.z0 + k};
-      const int bs[3] = {t.bx, t.by, t.bz};
-      const int v0 = gi[D0] == 0 ? -1 : (gi[D0] == bs[D0] ? 1 : 0);
-      const int v1 = (C::DIM == 2 && D1 == 2) ? 0 : (gi[D1] == 0 ? -1 : (gi[D1] == bs[D1] ? 1 : 0));
-      if constexpr (C::AMR)
-        out = amr_border_emf<C, CD, D0, D1>(t, gi, v0, v1, val);
-      else if (v0 != 0 && v1 != 0)
+    edge_states<C, CD>(t, i, j, k, qe);
+    store_emf<C, CD>(t, i, j, k, edge_emf<R, CD>(qe, t.ph) * t.dtdx);
+  }
+}
+
+// The same on the FP64 path: all directions in one list, so that the solver's code (long: divisions and square roots
+// are integer sequences) is in the kernel once. With a copy for each direction the warps of a CTA, spread over the
+// passes, missed the instruction cache: 5.5 of 15 stalled cycles per instruction on 3D Orszag-Tang.
+template <class C>
+__device__ __forceinline__ void
+edge_pass_fp64(const TileView<C> & t, int tid)
+{
+#pragma unroll 1
+  for (int m = tid; m < C::NEDGE; m += C::NT)
+  {
+    int    i, j, k;
+    double r[4], p[4], u[4], v[4], c[4], a0, a1, b0, b1;
+    auto   states = [&](auto dir, int n) {
+      constexpr int CD = decltype(dir)::value;
+      constexpr int NX = CD == 0 ? C::TX : C::TX + 1, NY = CD == 1 ? C::TY : C::TY + 1;
+      // (u, v) and (a, b) the edge's transverse axes in turn, c along it
+      constexpr int iu = CD == 2 ? IU : (CD == 1 ? IW : IV), iv = CD == 2 ? IV : (CD == 1 ? IU : IW);
+      constexpr int ia = iu + 3, ib = iv + 3, ic = CD == 2 ? IC : (CD == 1 ? IB : IA);
+      i = n % NX;
+      j = (n / NX) % NY;
+      k = n / (NX * NY);
+      double qe[4][8];
+      edge_states<C, CD>(t, i, j, k, qe);
+      const double * st[4] = {qe[ERT], qe[ERB], qe[ELT], qe[ELB]};
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
       {
-        const int sl0 = nb_slot(D0 == 0 ? v0 : 0, D0 == 1 ? v0 : 0, 0);
-        const int sl1 = nb_slot(D1 == 0 ? v1 : 0, D1 == 1 ? v1 : 0, D1 == 2 ? v1 : 0);
-        const int sl2 = nb_slot(D0 == 0 ? v0 : (D1 == 0 ? v1 : 0), D0 == 1 ? v0 : (D1 == 1 ? v1 : 0), D1 == 2 ? v1 : 0);
-        const int n0 = t.s_nbr[sl0], n1 = t.s_nbr[sl1], n2 = t.s_nbr[sl2];
-        if (n0 >= 0 && n1 >= 0 && n2 >= 0)
-        {
-          R   acc = R(0);
-          int count = 1;
-          acc += val;
-          if (n0 < t.n_owned)
-          {
-            acc += val;
-            count++;
-          }
-          if (n1 < t.n_owned)
-          {
-            acc += val;
-            count++;
-          }
-          if (n2 < t.n_owned)
-          {
-            acc += val;
-            count++;
-          }
-          val = acc / (R)count;
-        }
+        r[q] = st[q][ID];
+        p[q] = st[q][IP];
+        u[q] = st[q][iu];
+        v[q] = st[q][iv];
+        c[q] = st[q][ic];
       }
-      if constexpr (!C::AMR)
-        out = to_d<R>(val);
+      a0 = qe[ERT][ia] + qe[ELT][ia];
+      a1 = qe[ERB][ia] + qe[ELB][ia];
+      b0 = qe[ERT][ib] + qe[ERB][ib];
+      b1 = qe[ELT][ib] + qe[ELB][ib];
+    };
+    if (C::DIM == 2 || m < C::NEZ)
+      states(std::integral_constant<int, 2>{}, m);
+    else if constexpr (C::DIM == 3)
+    {
+      if (m < C::NEZ + C::NEY)
+        states(std::integral_constant<int, 1>{}, m - C::NEZ);
+      else
+        states(std::integral_constant<int, 0>{}, m - C::NEZ - C::NEY);
     }
-    t.emfd[(C::DIM == 3 ? CD : 0) * C::NM + C::mi(i, j, k)] = out;
+    const double val = edge_emf_fp64(r, p, u, v, c, dscale_down(a0, 1), dscale_down(a1, 1), dscale_down(b0, 1),
+                                     dscale_down(b1, 1), t.ph.gamma0, t.ph.smallc) *
+                       t.dtdx;
+    if (C::DIM == 2 || m < C::NEZ)
+      store_emf<C, 2>(t, i, j, k, val);
+    else if constexpr (C::DIM == 3)
+    {
+      if (m < C::NEZ + C::NEY)
+        store_emf<C, 1>(t, i, j, k, val);
+      else
+        store_emf<C, 0>(t, i, j, k, val);
+    }
   }
 }
 
@@ -806,8 +892,8 @@ flux_pass(const TileView<C> & t, int tid)
 #pragma unroll
     for (int v = 0; v < 8; ++v)
     {
-      qL[v] = t.q2[v * NS + snL] + R(0.5) * S[v * NS + snL];
-      qR[v] = t.q2[v * NS + snR] + R(-0.5) * S[v * NS + snR];
+      qL[v] = plus_half<R>(t.q2[v * NS + snL], S[v * NS + snL]);
+      qR[v] = minus_half<R>(t.q2[v * NS + snR], S[v * NS + snR]);
     }
     qL[ID] = rmax<R>(t.ph.smallr, qL[ID]);
     qL[IP] = rmax<R>(t.ph.smallp * qL[ID], qL[IP]);
@@ -836,6 +922,59 @@ flux_pass(const TileView<C> & t, int tid)
       t.fl[v * C::NFT + OFF + m] = flux[v] * t.dtdx;
     if constexpr (C::DIM == 2)
       t.fl[5 * C::NFT + OFF + m] = flux[IC] * t.dtdx;
+  }
+}
+
+// The same on the FP64 path: all directions in one list (see edge_pass_fp64)
+template <class C>
+__device__ __forceinline__ void
+flux_pass_fp64(const TileView<C> & t, int tid)
+{
+  constexpr int NS = C::NS;
+#pragma unroll 1
+  for (int m = first_item<C>(tid, C::NEDGE % C::NT); m < C::NFT; m += C::NT)
+  {
+    const int d = m < C::NF_X ? 0 : (m < C::NF_X + C::NF_Y ? 1 : 2);
+    const int n = m - (d == 0 ? 0 : (d == 1 ? C::NF_X : C::NF_X + C::NF_Y));
+    const int nx = C::TX + (d == 0), ny = C::TY + (d == 1);
+    const int k = n / (nx * ny), j = (n - k * nx * ny) / nx, i = n - (k * ny + j) * nx;
+    const int snR = C::si(i, j, k);
+    const int snL = snR - (d == 0 ? s_stride<C>(0) : (d == 1 ? s_stride<C>(1) : s_stride<C>(2)));
+    const double * S = t.sl + d * 8 * NS;
+    double         qL[8], qR[8], flux[8];
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+    {
+      qL[v] = fma(0.5, S[v * NS + snL], t.q2[v * NS + snL]);
+      qR[v] = fma(-0.5, S[v * NS + snR], t.q2[v * NS + snR]);
+    }
+    qL[ID] = dmax(t.ph.smallr, qL[ID]);
+    qL[IP] = dmax(t.ph.smallp * qL[ID], qL[IP]);
+    qR[ID] = dmax(t.ph.smallr, qR[ID]);
+    qR[IP] = dmax(t.ph.smallp * qR[ID], qR[IP]);
+    const int    fi = d == 0 ? C::fxi(i, j, k) : (d == 1 ? C::fyi(i, j, k) : C::fzi(i, j, k));
+    const double bn = (d == 0 ? t.fb[0] : (d == 1 ? t.fb[1] : t.fb[2]))[fi] + t.sf[d * NS + snR];
+    // the normal components first
+    auto turn = [&](double * q) {
+      const double u = q[IU], a = q[IA];
+      q[IU] = d == 0 ? q[IU] : (d == 1 ? q[IV] : q[IW]);
+      q[IV] = d == 1 ? u : q[IV];
+      q[IW] = d == 2 ? u : q[IW];
+      q[IA] = d == 0 ? q[IA] : (d == 1 ? q[IB] : q[IC]);
+      q[IB] = d == 1 ? a : q[IB];
+      q[IC] = d == 2 ? a : q[IC];
+    };
+    turn(qL);
+    turn(qR);
+    qL[IA] = bn;
+    qR[IA] = bn;
+    riemann_mhd<double>(qL, qR, flux, t.ph);
+    turn(flux);
+#pragma unroll
+    for (int v = 0; v < 5; ++v)
+      t.fl[v * C::NFT + m] = flux[v] * t.dtdx;
+    if constexpr (C::DIM == 2)
+      t.fl[5 * C::NFT + m] = flux[IC] * t.dtdx;
   }
 }
 
@@ -1184,6 +1323,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
     ph.smallc = a.smallc;
     ph.smallp = a.smallp;
     ph.slope_type = a.slope_type;
+    ph.entho = a.entho;
   }
   ph.riemann = a.riemann;
 
@@ -1446,10 +1586,9 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
     if constexpr (C::EXACT)
     {
       // compute_primitives (models/mhd_utils.h:449-515), cIso == 0
-      double Bxc = 0.5 * (fbx[C::fxi(i, j, k)] + fbx[C::fxi(i + 1, j, k)]);
-      double Byc = 0.5 * (fby[C::fyi(i, j, k)] + fby[C::fyi(i, j + 1, k)]);
-      double Bzc = D3 ? 0.5 * (fbz[C::fzi(i, j, k)] + fbz[C::fzi(i, j, k + 1)])
-                      : 0.5 * (fbz[C::fzi(i, j, 0)] + fbz[C::fzi(i, j, 0)]);
+      double Bxc = dscale_down(fbx[C::fxi(i, j, k)] + fbx[C::fxi(i + 1, j, k)], 1);
+      double Byc = dscale_down(fby[C::fyi(i, j, k)] + fby[C::fyi(i, j + 1, k)], 1);
+      double Bzc = D3 ? dscale_down(fbz[C::fzi(i, j, k)] + fbz[C::fzi(i, j, k + 1)], 1) : fbz[C::fzi(i, j, 0)];
       if (coarse_copy || has_outside)
       {
         double bc[3];
@@ -1460,12 +1599,12 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
           Bzc = bc[2];
         }
       }
-      const double r = fmax(u[ID], a.smallr);
-      const double vx = u[IU] / r, vy = u[IV] / r, vz = u[IW] / r;
-      const double eken = 0.5 * (vx * vx + vy * vy + vz * vz);
-      const double emag = 0.5 * (Bxc * Bxc + Byc * Byc + Bzc * Bzc);
-      const double eint = (u[IP] - emag) / r - eken;
-      const double p = fmax((a.gamma0 - 1.0) * r * eint, r * a.smallp);
+      const double r = dmax(u[ID], a.smallr);
+      const Rcp64  ir = rcp64(r);
+      const double vx = div64(u[IU], ir), vy = div64(u[IV], ir), vz = div64(u[IW], ir);
+      const double eint = fma(-0.5, vx * vx + vy * vy + vz * vz,
+                              div64(fma(-0.5, Bxc * Bxc + Byc * Byc + Bzc * Bzc, u[IP]), ir));
+      const double p = dmax((a.gamma0 - 1.0) * r * eint, r * a.smallp);
       qh[0 * C::NQ + qn] = r;
       qh[1 * C::NQ + qn] = p;
       qh[2 * C::NQ + qn] = vx;
@@ -1618,11 +1757,11 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
     const R BL = fby[C::fyi(i, j, k)], BR = fby[C::fyi(i, j + 1, k)];
     const R CL = D3 ? fbz[C::fzi(i, j, k)] : fbz[C::fzi(i, j, 0)];
     const R CR = D3 ? fbz[C::fzi(i, j, k + 1)] : fbz[C::fzi(i, j, 0)];
-    auto    avgA = [&](int ii, int jj, int kk) { return (fbx[C::fxi(ii, jj, kk)] + fbx[C::fxi(ii + 1, jj, kk)]) * R(0.5); };
-    auto    avgB = [&](int ii, int jj, int kk) { return (fby[C::fyi(ii, jj, kk)] + fby[C::fyi(ii, jj + 1, kk)]) * R(0.5); };
+    auto    avgA = [&](int ii, int jj, int kk) { return half_of<R>(fbx[C::fxi(ii, jj, kk)] + fbx[C::fxi(ii + 1, jj, kk)]); };
+    auto    avgB = [&](int ii, int jj, int kk) { return half_of<R>(fby[C::fyi(ii, jj, kk)] + fby[C::fyi(ii, jj + 1, kk)]); };
     auto    avgC = [&](int ii, int jj, int kk) {
-      return D3 ? (fbz[C::fzi(ii, jj, kk)] + fbz[C::fzi(ii, jj, kk + 1)]) * R(0.5)
-                : (fbz[C::fzi(ii, jj, 0)] + fbz[C::fzi(ii, jj, 0)]) * R(0.5);
+      return D3 ? half_of<R>(fbz[C::fzi(ii, jj, kk)] + fbz[C::fzi(ii, jj, kk + 1)])
+                : half_of<R>(fbz[C::fzi(ii, jj, 0)] + fbz[C::fzi(ii, jj, 0)]);
     };
     dq[0][IA] = AR - AL;
     dq[1][IA] = slope1<R>(avgA(i, j, k), avgA(i, j + 1, k), avgA(i, j - 1, k), st);
@@ -1649,7 +1788,14 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
     // Hancock predictor
     const R r = qh[0 * C::NQ + q0], p = qh[1 * C::NQ + q0], u = qh[2 * C::NQ + q0],
             v = qh[3 * C::NQ + q0], w = qh[4 * C::NQ + q0];
-    const R A = (AL + AR) * R(0.5), B = (BL + BR) * R(0.5), Cc = (CL + CR) * R(0.5);
+    const R A = half_of<R>(AL + AR), B = half_of<R>(BL + BR), Cc = half_of<R>(CL + CR);
+    const auto ir = recip<R>(r); // FP64 path
+    auto       by_r = [&](R x) -> R {
+      if constexpr (C::EXACT)
+        return div64(x, ir);
+      else
+        return x / r;
+    };
     if (a.rk2)
     {
       // RK2_SSP: Q2 = Q (ComputeUpdatedPrimitiveVariablesFunctor.cpp:396-407, 531-542)
@@ -1673,9 +1819,9 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
     if constexpr (DIM == 2)
     {
       sr0 = (-u * drx - dux * r) * dtdx + (-v * dry - dvy * r) * dtdy;
-      su0 = (-u * dux - dpx / r - B * dBx / r - Cc * dCx / r) * dtdx + (-v * duy + B * dAy / r) * dtdy;
-      sv0 = (-u * dvx + A * dBx / r) * dtdx + (-v * dvy - dpy / r - A * dAy / r - Cc * dCy / r) * dtdy;
-      sw0 = (-u * dwx + A * dCx / r) * dtdx + (-v * dwy + B * dCy / r) * dtdy;
+      su0 = (-u * dux - by_r(dpx) - by_r(B * dBx) - by_r(Cc * dCx)) * dtdx + (-v * duy + by_r(B * dAy)) * dtdy;
+      sv0 = (-u * dvx + by_r(A * dBx)) * dtdx + (-v * dvy - by_r(dpy) - by_r(A * dAy) - by_r(Cc * dCy)) * dtdy;
+      sw0 = (-u * dwx + by_r(A * dCx)) * dtdx + (-v * dwy + by_r(B * dCy)) * dtdy;
       sp0 = (-u * dpx - dux * gamma * p) * dtdx + (-v * dpy - dvy * gamma * p) * dtdy;
       sA0 = (u * dBy + B * duy - v * dAy - A * dvy) * dtdy;
       sB0 = (-u * dBx - B * dux + v * dAx + A * dvx) * dtdx;
@@ -1686,12 +1832,12 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
       const R drz = dq[2][ID], dpz = dq[2][IP], duz = dq[2][IU], dvz = dq[2][IV], dwz = dq[2][IW],
               dAz = dq[2][IA], dBz = dq[2][IB], dCz = dq[2][IC];
       sr0 = (-u * drx - dux * r) * dtdx + (-v * dry - dvy * r) * dtdy + (-w * drz - dwz * r) * dtdz;
-      su0 = (-u * dux - (dpx + B * dBx + Cc * dCx) / r) * dtdx + (-v * duy + B * dAy / r) * dtdy +
-            (-w * duz + Cc * dAz / r) * dtdz;
-      sv0 = (-u * dvx + A * dBx / r) * dtdx + (-v * dvy - (dpy + A * dAy + Cc * dCy) / r) * dtdy +
-            (-w * dvz + Cc * dBz / r) * dtdz;
-      sw0 = (-u * dwx + A * dCx / r) * dtdx + (-v * dwy + B * dCy / r) * dtdy +
-            (-w * dwz - (dpz + A * dAz + B * dBz) / r) * dtdz;
+      su0 = (-u * dux - by_r(dpx + B * dBx + Cc * dCx)) * dtdx + (-v * duy + by_r(B * dAy)) * dtdy +
+            (-w * duz + by_r(Cc * dAz)) * dtdz;
+      sv0 = (-u * dvx + by_r(A * dBx)) * dtdx + (-v * dvy - by_r(dpy + A * dAy + Cc * dCy)) * dtdy +
+            (-w * dvz + by_r(Cc * dBz)) * dtdz;
+      sw0 = (-u * dwx + by_r(A * dCx)) * dtdx + (-v * dwy + by_r(B * dCy)) * dtdy +
+            (-w * dwz - by_r(dpz + A * dAz + B * dBz)) * dtdz;
       sp0 = (-u * dpx - dux * gamma * p) * dtdx + (-v * dpy - dvy * gamma * p) * dtdy +
             (-w * dpz - dwz * gamma * p) * dtdz;
       sA0 = (u * dBy + B * duy - v * dAy - A * dvy) * dtdy + (u * dCz + Cc * duz - w * dAz - A * dwz) * dtdz;
@@ -1714,18 +1860,25 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
       if (a.src.visc_predictor)
       {
         // (ComputeUpdatedPrimitiveVariablesFunctor.cpp:174-280): half a step of nu * Laplacian per axis
-        const R nu = (R)a.src.mu / r;
+        const R nu = by_r((R)a.src.mu);
+        const auto idx = recip<R>(dxr);
+        auto       over_dx = [&](R x) -> R {
+          if constexpr (C::EXACT)
+            return div64(x, idx);
+          else
+            return x / dxr;
+        };
         auto    vp = [&](int var, R val) {
           const R * Q = qh + var * C::NQ;
           const R   q0v = Q[q0];
           const R   d2x = Q[qxp] + Q[qxm] - R(2) * q0v;
-          val += R(0.5) * nu * d2x / dxr * dtdx;
+          val += over_dx(R(0.5) * nu * d2x) * dtdx;
           const R d2y = Q[qyp] + Q[qym] - R(2) * q0v;
-          val += R(0.5) * nu * d2y / dxr * dtdx;
+          val += over_dx(R(0.5) * nu * d2y) * dtdx;
           if constexpr (DIM == 3)
           {
             const R d2z = Q[qzp] + Q[qzm] - R(2) * q0v;
-            val += R(0.5) * nu * d2z / dxr * dtdx;
+            val += over_dx(R(0.5) * nu * d2z) * dtdx;
           }
           return val;
         };
@@ -1735,14 +1888,14 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
           wg = vp(IW, wg);
       }
     }
-    q2[ID * C::NS + n] = r + R(0.5) * sr0;
-    q2[IU * C::NS + n] = ug + R(0.5) * su0;
-    q2[IV * C::NS + n] = vg + R(0.5) * sv0;
-    q2[IW * C::NS + n] = wg + R(0.5) * sw0;
-    q2[IP * C::NS + n] = p + R(0.5) * sp0;
-    q2[IA * C::NS + n] = A + R(0.5) * sA0;
-    q2[IB * C::NS + n] = B + R(0.5) * sB0;
-    q2[IC * C::NS + n] = Cc + R(0.5) * sC0;
+    q2[ID * C::NS + n] = plus_half<R>(r, sr0);
+    q2[IU * C::NS + n] = plus_half<R>(ug, su0);
+    q2[IV * C::NS + n] = plus_half<R>(vg, sv0);
+    q2[IW * C::NS + n] = plus_half<R>(wg, sw0);
+    q2[IP * C::NS + n] = plus_half<R>(p, sp0);
+    q2[IA * C::NS + n] = plus_half<R>(A, sA0);
+    q2[IB * C::NS + n] = plus_half<R>(B, sB0);
+    q2[IC * C::NS + n] = plus_half<R>(Cc, sC0);
   }
 
   // ---- phase 3: edge electric field at t^n on [-1, T+2) (ComputeElectricFieldFunctor.cpp:97-235)
@@ -1754,7 +1907,26 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
     const R * QU = qh + 2 * C::NQ;
     const R * QV = qh + 3 * C::NQ;
     const R * QW = qh + 4 * C::NQ;
-    if constexpr (DIM == 2)
+    if constexpr (C::EXACT)
+    {
+      // 8 E: the means' factors 1/4 and 1/2 are left to phase 4's factor (powers of two: the same bits there)
+      const R uz = ((QU[C::qi(i - 1, j - 1, k)] + QU[C::qi(i - 1, j, k)]) + QU[C::qi(i, j - 1, k)]) + QU[C::qi(i, j, k)];
+      const R vz = ((QV[C::qi(i - 1, j - 1, k)] + QV[C::qi(i - 1, j, k)]) + QV[C::qi(i, j - 1, k)]) + QV[C::qi(i, j, k)];
+      const R ez = uz * (fby[C::fyi(i - 1, j, k)] + fby[C::fyi(i, j, k)]) - vz * (fbx[C::fxi(i, j - 1, k)] + fbx[C::fxi(i, j, k)]);
+      if constexpr (DIM == 2)
+        ee[n] = ez;
+      else
+      {
+        const R vx = ((QV[C::qi(i, j - 1, k - 1)] + QV[C::qi(i, j - 1, k)]) + QV[C::qi(i, j, k - 1)]) + QV[C::qi(i, j, k)];
+        const R wx = ((QW[C::qi(i, j - 1, k - 1)] + QW[C::qi(i, j - 1, k)]) + QW[C::qi(i, j, k - 1)]) + QW[C::qi(i, j, k)];
+        const R uy = ((QU[C::qi(i - 1, j, k - 1)] + QU[C::qi(i - 1, j, k)]) + QU[C::qi(i, j, k - 1)]) + QU[C::qi(i, j, k)];
+        const R wy = ((QW[C::qi(i - 1, j, k - 1)] + QW[C::qi(i - 1, j, k)]) + QW[C::qi(i, j, k - 1)]) + QW[C::qi(i, j, k)];
+        ee[0 * C::NE + n] = vx * (fbz[C::fzi(i, j - 1, k)] + fbz[C::fzi(i, j, k)]) - wx * (fby[C::fyi(i, j, k - 1)] + fby[C::fyi(i, j, k)]);
+        ee[1 * C::NE + n] = wy * (fbx[C::fxi(i, j, k - 1)] + fbx[C::fxi(i, j, k)]) - uy * (fbz[C::fzi(i - 1, j, k)] + fbz[C::fzi(i, j, k)]);
+        ee[2 * C::NE + n] = ez;
+      }
+    }
+    else if constexpr (DIM == 2)
     {
       const R u = R(0.25) * (QU[C::qi(i - 1, j - 1, 0)] + QU[C::qi(i - 1, j, 0)] + QU[C::qi(i, j - 1, 0)] + QU[C::qi(i, j, 0)]);
       const R v = R(0.25) * (QV[C::qi(i - 1, j - 1, 0)] + QV[C::qi(i - 1, j, 0)] + QV[C::qi(i, j - 1, 0)] + QV[C::qi(i, j, 0)]);
@@ -1796,7 +1968,27 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
     const int j = (n / C::SX) % C::SY - 1;
     const int k = D3 ? n / (C::SX * C::SY) - 1 : 0;
     const R   dtdy = dtdx, dtdz = dtdx;
-    if constexpr (DIM == 2)
+    if constexpr (C::EXACT)
+    {
+      const R   h = R(0.0625) * dtdx; // 1/2 dt/dx, and 1/8 for the edge field (exact powers of two)
+      const R * Ez = ee + (DIM == 3 ? 2 * C::NE : 0);
+      const R   z0 = Ez[C::ei(i, j, k)], zy = (Ez[C::ei(i, j + 1, k)] - z0) * h, zx = (Ez[C::ei(i + 1, j, k)] - z0) * h;
+      if constexpr (DIM == 2)
+      {
+        sf[0 * C::NS + n] = zy;
+        sf[1 * C::NS + n] = -zx;
+      }
+      else
+      {
+        const R * Ex = ee;
+        const R * Ey = ee + C::NE;
+        const R   x0 = Ex[C::ei(i, j, k)], y0 = Ey[C::ei(i, j, k)];
+        sf[0 * C::NS + n] = zy - (Ey[C::ei(i, j, k + 1)] - y0) * h;
+        sf[1 * C::NS + n] = (Ex[C::ei(i, j, k + 1)] - x0) * h - zx;
+        sf[2 * C::NS + n] = (Ey[C::ei(i + 1, j, k)] - y0) * h - (Ex[C::ei(i, j + 1, k)] - x0) * h;
+      }
+    }
+    else if constexpr (DIM == 2)
     {
       sf[0 * C::NS + n] = (ee[C::ei(i, j + 1, 0)] - ee[C::ei(i, j, 0)]) * R(0.5) * dtdy;
       sf[1 * C::NS + n] = -(ee[C::ei(i + 1, j, 0)] - ee[C::ei(i, j, 0)]) * R(0.5) * dtdx;
@@ -1854,16 +2046,24 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
     constexpr int E1 = DIM == 3 ? edge_count<C, 1>() : 0;
     constexpr int E0 = DIM == 3 ? edge_count<C, 0>() : 0;
     constexpr int F0 = face_count<C, 0>(), F1 = face_count<C, 1>();
-    edge_pass<C, 2, 0>(tv, tid);
-    if constexpr (DIM == 3)
+    if constexpr (C::EXACT)
     {
-      edge_pass<C, 1, E2 % NT>(tv, tid);
-      edge_pass<C, 0, (E2 + E1) % NT>(tv, tid);
+      edge_pass_fp64<C>(tv, tid);
+      flux_pass_fp64<C>(tv, tid);
     }
-    flux_pass<C, 0, (E2 + E1 + E0) % NT>(tv, tid);
-    flux_pass<C, 1, (E2 + E1 + E0 + F0) % NT>(tv, tid);
-    if constexpr (DIM == 3)
-      flux_pass<C, 2, (E2 + E1 + E0 + F0 + F1) % NT>(tv, tid);
+    else
+    {
+      edge_pass<C, 2, 0>(tv, tid);
+      if constexpr (DIM == 3)
+      {
+        edge_pass<C, 1, E2 % NT>(tv, tid);
+        edge_pass<C, 0, (E2 + E1) % NT>(tv, tid);
+      }
+      flux_pass<C, 0, (E2 + E1 + E0) % NT>(tv, tid);
+      flux_pass<C, 1, (E2 + E1 + E0 + F0) % NT>(tv, tid);
+      if constexpr (DIM == 3)
+        flux_pass<C, 2, (E2 + E1 + E0 + F0 + F1) % NT>(tv, tid);
+    }
   }
   __syncthreads();
   if constexpr (C::AMR)
@@ -1960,9 +2160,9 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
         const int i = n % (TX + 1), j = (n / (TX + 1)) % TY, k = n / ((TX + 1) * TY);
         double d;
         if constexpr (DIM == 2)
-          d = curl2<C::EXACT>(Mz[C::mi(i, j + 1, 0)] - Mz[C::mi(i, j, 0)], 0.0);
+          d = Mz[C::mi(i, j + 1, 0)] - Mz[C::mi(i, j, 0)];
         else
-          d = curl2<C::EXACT>(Mz[C::mi(i, j + 1, k)] - Mz[C::mi(i, j, k)], My[C::mi(i, j, k + 1)] - My[C::mi(i, j, k)]);
+          d = curl2(Mz[C::mi(i, j + 1, k)] - Mz[C::mi(i, j, k)], My[C::mi(i, j, k + 1)] - My[C::mi(i, j, k)]);
         bnew = bold[it] + d;
         owned = i < TX || ex;
       }
@@ -1975,7 +2175,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
         else
         {
           const double d =
-            curl2<C::EXACT>(Mx[C::mi(i, j, k + 1)] - Mx[C::mi(i, j, k)], Mz[C::mi(i + 1, j, k)] - Mz[C::mi(i, j, k)]);
+            curl2(Mx[C::mi(i, j, k + 1)] - Mx[C::mi(i, j, k)], Mz[C::mi(i + 1, j, k)] - Mz[C::mi(i, j, k)]);
           bnew = bold[it] + d;
         }
         owned = j < TY || ey;
@@ -1985,7 +2185,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
         const int nn = n - C::NB2X - C::NB2Y;
         const int i = nn % TX, j = (nn / TX) % TY, k = nn / (TX * TY);
         const double d =
-          curl2<C::EXACT>(My[C::mi(i + 1, j, k)] - My[C::mi(i, j, k)], Mx[C::mi(i, j + 1, k)] - Mx[C::mi(i, j, k)]);
+          curl2(My[C::mi(i + 1, j, k)] - My[C::mi(i, j, k)], Mx[C::mi(i, j + 1, k)] - Mx[C::mi(i, j, k)]);
         bnew = bold[it] + d;
         owned = k < TZ || ez;
       }
@@ -2043,10 +2243,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
       {
         if constexpr (C::EXACT)
         {
-          R acc = R(0);
-          acc = acc + fl[v * C::NFT + fL];
-          acc = acc - fl[v * C::NFT + fR];
-          u2[v] += (double)acc;
+          u2[v] += fl[v * C::NFT + fL] - fl[v * C::NFT + fR]; // (0 + left) - right: the same up to a zero's sign
         }
         else
         {
@@ -2164,20 +2361,21 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
       // AddGravitySourceTerm (AddGravitySourceTerm.cpp:47-99), FP64
       const double rho_old = upre[c][ID], rho_new = u2[ID];
       double       ru = u2[IU], rv = u2[IV], rw = DIM == 3 ? u2[IW] : 0.0;
-      double       ekin_old = 0.5 * (ru * ru + rv * rv) / rho_new;
+      const Rcp64  irn = rcp64(rho_new);
+      double       ekin_old = div64(dscale_down(ru * ru + rv * rv, 1), irn);
       if constexpr (DIM == 3)
-        ekin_old += 0.5 * (rw * rw) / rho_new;
-      ru += dt * a.src.g[0] * (rho_old + rho_new) / 2;
-      rv += dt * a.src.g[1] * (rho_old + rho_new) / 2;
+        ekin_old += div64(dscale_down(rw * rw, 1), irn);
+      ru += dscale_down(dt * a.src.g[0] * (rho_old + rho_new), 1);
+      rv += dscale_down(dt * a.src.g[1] * (rho_old + rho_new), 1);
       if constexpr (DIM == 3)
-        rw += dt * a.src.g[2] * (rho_old + rho_new) / 2;
+        rw += dscale_down(dt * a.src.g[2] * (rho_old + rho_new), 1);
       u2[IU] = ru;
       u2[IV] = rv;
       if constexpr (DIM == 3)
         u2[IW] = rw;
-      double ekin_new = 0.5 * (ru * ru + rv * rv) / rho_new;
+      double ekin_new = div64(dscale_down(ru * ru + rv * rv, 1), irn);
       if constexpr (DIM == 3)
-        ekin_new += 0.5 * (rw * rw) / rho_new;
+        ekin_new += div64(dscale_down(rw * rw, 1), irn);
       u2[IP] += (ekin_new - ekin_old);
     }
 #pragma unroll
@@ -2202,28 +2400,14 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
       [[maybe_unused]] double val = 0.0; // FP64 path
       if constexpr (C::EXACT)
       {
-        const double Ax = 0.5 * (Axl + Axr);
-        const double Ay = 0.5 * (Ayl + Ayr);
+        const double Ax = dscale_down(Axl + Axr, 1);
+        const double Ay = dscale_down(Ayl + Ayr, 1);
         double       Az;
         if constexpr (DIM == 3)
-          Az = 0.5 * (b2s[C::NB2X + C::NB2Y + i + TX * (j + TY * k)] + b2s[C::NB2X + C::NB2Y + i + TX * (j + TY * (k + 1))]);
+          Az = dscale_down(b2s[C::NB2X + C::NB2Y + i + TX * (j + TY * k)] + b2s[C::NB2X + C::NB2Y + i + TX * (j + TY * (k + 1))], 1);
         else
-          Az = 0.5 * (u2[5] + u2[5]);
-        const double r = fmax(u2[ID], a.smallr);
-        const double vx = u2[IU] / r, vy = u2[IV] / r, vz = u2[IW] / r;
-        const double eken = 0.5 * (vx * vx + vy * vy + vz * vz);
-        const double emag = 0.5 * (Ax * Ax + Ay * Ay + Az * Az);
-        const double eint = (u2[IP] - emag) / r - eken;
-        const double p = fmax((a.gamma0 - 1.0) * r * eint, r * a.smallp);
-        const double b2 = Ax * Ax + Ay * Ay + Az * Az;
-        const double c2 = a.gamma0 * p / r;
-        const double d2 = 0.5 * (b2 / r + c2);
-        const double cfx = sqrt(d2 + sqrt(d2 * d2 - c2 * Ax * Ax / r)) + fabs(vx);
-        const double cfy = sqrt(d2 + sqrt(d2 * d2 - c2 * Ay * Ay / r)) + fabs(vy);
-        double cfz = 0.0;
-        if constexpr (DIM == 3)
-          cfz = sqrt(d2 + sqrt(d2 * d2 - c2 * Az * Az / r)) + fabs(vz);
-        val = cfl_inv_dt_fp64(DIM, cfx, cfy, cfz, dx, u2[ID], a.src);
+          Az = u2[5];
+        val = cell_inv_dt_fp64(u2, Ax, Ay, Az, DIM, dx, a.gamma0, a.smallr, a.smallp, a.src);
       }
       else
       {

@@ -343,6 +343,15 @@ sources_of(const gmhd_params & p)
   return src;
 }
 
+// the tile request passed to the launchers: the context's, or the default for a mesh of few tiles
+int
+tile_request(const gmhd_ctx * c)
+{
+  if (c->tile || c->p.precision == GMHD_PRECISION_MIXED)
+    return c->tile;
+  return gmhd::default_tile_fp64(c->dim, c->bx, c->by, c->bz, c->n_owned);
+}
+
 gmhd::StepArgs
 make_args(const gmhd_ctx * c, const double * U, double * U2, const double * B, double * B2)
 {
@@ -356,7 +365,7 @@ make_args(const gmhd_ctx * c, const double * U, double * U2, const double * B, d
   a.level = c->d_level;
   a.problem = c->d_problem;
   a.n_owned = c->n_owned;
-  a.tile = c->tile;
+  a.tile = tile_request(c);
   a.bx = c->bx;
   a.by = c->by;
   a.bz = c->bz;
@@ -368,6 +377,7 @@ make_args(const gmhd_ctx * c, const double * U, double * U2, const double * B, d
   a.smallr = c->p.smallr;
   a.smallc = c->p.smallc;
   a.smallp = c->smallp;
+  a.entho = 1.0 / (c->p.gamma0 - 1.0);
   a.slope_type = c->p.slope_type;
   a.scaling_factor = c->p.scaling_factor;
   a.cfl = c->p.cfl;
@@ -746,7 +756,7 @@ build_tile_lists(gmhd_ctx * ctx, int dim, const std::vector<int8_t> & kind)
   if (ctx->p.precision == GMHD_PRECISION_MIXED)
     gmhd::tile_shape_mixed(dim, ctx->bx, ctx->by, ctx->bz, ctx->p.viscosity_enabled != 0, true, ctx->tile, T);
   else
-    gmhd::tile_shape_fp64(dim, ctx->bx, ctx->by, ctx->bz, ctx->p.viscosity_enabled != 0, ctx->tile, T);
+    gmhd::tile_shape_fp64(dim, ctx->bx, ctx->by, ctx->bz, ctx->p.viscosity_enabled != 0, tile_request(ctx), T);
   const int              nt[3] = {ctx->bx / T[0], ctx->by / T[1], dim == 3 ? ctx->bz / T[2] : 1};
   const int              tpb = nt[0] * nt[1] * nt[2];
   std::vector<int32_t> & list1 = ctx->h_list1;
@@ -1649,7 +1659,7 @@ plan_host_tiles(gmhd_ctx * ctx)
   if (mixed)
     gmhd::tile_shape_mixed(ctx->dim, ctx->bx, ctx->by, ctx->bz, visc, false, ctx->tile, T);
   else
-    gmhd::tile_shape_fp64(ctx->dim, ctx->bx, ctx->by, ctx->bz, visc, ctx->tile, T);
+    gmhd::tile_shape_fp64(ctx->dim, ctx->bx, ctx->by, ctx->bz, visc, tile_request(ctx), T);
   const int key = (T[0] << 16) | (T[1] << 8) | T[2];
   if (key == ctx->hp_tile_key)
     return GMHD_OK;

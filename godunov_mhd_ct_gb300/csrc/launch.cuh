@@ -8,6 +8,8 @@
 namespace gmhd
 {
 
+constexpr int kSMs = 152;
+
 // Launch the fused step for configuration C. Returns a cudaError_t (0 on success) or -1 when the
 // tile does not divide the block.
 // Resident CTAs of configuration C on the whole device (persistent variants), set by prepare_fused.
@@ -79,6 +81,9 @@ int tile_candidates_mixed(int dim, int bx, int by, int bz, bool visc, bool amr, 
 // the tile extents launch_step_* uses for these block sizes and request (column step: 16, 8, bz)
 void tile_shape_fp64(int dim, int bx, int by, int bz, bool visc, int tile, int * t);
 void tile_shape_mixed(int dim, int bx, int by, int bz, bool visc, bool amr, int tile, int * t);
+// the tile the FP64 step takes when none is asked for: a smaller one than the largest that divides the block (0)
+// where the mesh has too few tiles to occupy half the SMs, so that four or two tiles do the work of one
+int default_tile_fp64(int dim, int bx, int by, int bz, int n_owned);
 // column step (step_column.cu): -1 when it does not apply to these blocks / this mesh
 int launch_column(const StepArgs & a, cudaStream_t stream);
 int prepare_column();

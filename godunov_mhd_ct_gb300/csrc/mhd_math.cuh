@@ -8,6 +8,8 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "exact_solvers.cuh"
+
 namespace gmhd
 {
 
@@ -50,7 +52,8 @@ struct Sources
 __device__ __forceinline__ double
 cfl_inv_dt_fp64(int dim, double vx, double vy, double vz, double dx, double rho, const Sources & s)
 {
-  double val;
+  double      val;
+  const Rcp64 idx = rcp64(dx);
   if (s.gravity)
   {
     double v2 = vx * vx + vy * vy;
@@ -59,58 +62,70 @@ cfl_inv_dt_fp64(int dim, double vx, double vy, double vz, double dx, double rho,
     double k = fabs(s.g[0]) + fabs(s.g[1]);
     if (dim == 3)
       k += fabs(s.g[2]);
-    k *= dx / v2;
-    k = fmax(k, 1e-4);
-    const double factor = k / (sqrt(1.0 + 2.0 * k) - 1.0);
+    k *= div64(dx, v2);
+    k = dmax(k, 1e-4);
+    const double factor = div64(k, sqrt64(1.0 + 2.0 * k) - 1.0);
     val = 0.0;
-    val += (vx * factor) / dx;
-    val += (vy * factor) / dx;
+    val += div64(vx * factor, idx);
+    val += div64(vy * factor, idx);
     if (dim == 3)
-      val += (vz * factor) / dx;
+      val += div64(vz * factor, idx);
   }
   else
-    val = dim == 3 ? vx / dx + vy / dx + vz / dx : vx / dx + vy / dx;
+    val = dim == 3 ? div64(vx, idx) + div64(vy, idx) + div64(vz, idx) : div64(vx, idx) + div64(vy, idx);
   if (s.viscosity)
   {
-    const double nu = s.mu / rho;
-    val = fmax(val, 4 * nu / (dx * dx));
+    const double nu = div64(s.mu, rho);
+    val = dmax(val, div64(4 * nu, dx * dx));
   }
   return val;
 }
 
-// compute_cfl (scheme/ComputeDtMHDFunctor.cpp:86-151) of cell (i, j, k) of one block in the C-ABI
-// layout, FP64 with the reference operand order: face B averaged to the cell centre, primitive
-// recovery (models/mhd_utils.h:449-515), fast speeds (find_speed_info, :340-394), then
-// cfl_inv_dt_fp64. Ub / Bb point at the block's U and face arrays; c is the cell's index in the block.
+// The same from a cell's conservative state and cell-centred field: primitive recovery
+// (models/mhd_utils.h:449-515), fast speeds (find_speed_info, :340-394), then cfl_inv_dt_fp64.
 // Units that call it are compiled with --fmad=false, so every caller gets the same bits.
+__device__ __forceinline__ double
+cell_inv_dt_fp64(const double * u, double Ax, double Ay, double Az, int dim, double dx, double gamma0, double smallr,
+                 double smallp, const Sources & src)
+{
+  const double r = dmax(u[0], smallr);
+  const Rcp64  ir = rcp64(r);
+  const double vx = div64(u[2], ir), vy = div64(u[3], ir), vz = div64(u[4], ir);
+  const double b2 = Ax * Ax + Ay * Ay + Az * Az;
+  const double eint = fma(-0.5, vx * vx + vy * vy + vz * vz, div64(fma(-0.5, b2, u[1]), ir));
+  const double p = dmax((gamma0 - 1.0) * r * eint, r * smallp);
+  const double c2 = div64(gamma0 * p, ir);
+  const double d2 = dscale_down(div64(b2, ir) + c2, 1);
+  const double dd = d2 * d2;
+  const double cfx = sqrt64(d2 + sqrt64(dd - div64(c2 * Ax * Ax, ir))) + fabs(vx);
+  const double cfy = sqrt64(d2 + sqrt64(dd - div64(c2 * Ay * Ay, ir))) + fabs(vy);
+  const double cfz = dim == 3 ? sqrt64(d2 + sqrt64(dd - div64(c2 * Az * Az, ir))) + fabs(vz) : 0.0;
+  return cfl_inv_dt_fp64(dim, cfx, cfy, cfz, dx, u[0], src);
+}
+
+// compute_cfl (scheme/ComputeDtMHDFunctor.cpp:86-151) of cell (i, j, k) of one block in the C-ABI
+// layout, FP64 with the reference operand order: face B averaged to the cell centre, then the above.
+// Ub / Bb point at the block's U and face arrays; c is the cell's index in the block.
 __device__ __forceinline__ double
 cell_inv_dt_fp64(const double * __restrict__ Ub, const double * __restrict__ Bb, int dim, int bx, int by, int i,
                  int j, int k, int64_t c, int64_t ncell, int64_t nfx, int64_t nfy, double dx, double gamma0,
                  double smallr, double smallp, const Sources & src)
 {
-  const double Ax = 0.5 * (Bb[i + (int64_t)(bx + 1) * (j + (int64_t)by * k)] +
-                           Bb[i + 1 + (int64_t)(bx + 1) * (j + (int64_t)by * k)]);
-  const double Ay = 0.5 * (Bb[nfx + i + (int64_t)bx * (j + (int64_t)(by + 1) * k)] +
-                           Bb[nfx + i + (int64_t)bx * (j + 1 + (int64_t)(by + 1) * k)]);
+  const double Ax = dscale_down(Bb[i + (int64_t)(bx + 1) * (j + (int64_t)by * k)] +
+                                  Bb[i + 1 + (int64_t)(bx + 1) * (j + (int64_t)by * k)],
+                                1);
+  const double Ay = dscale_down(Bb[nfx + i + (int64_t)bx * (j + (int64_t)(by + 1) * k)] +
+                                  Bb[nfx + i + (int64_t)bx * (j + 1 + (int64_t)(by + 1) * k)],
+                                1);
   double Az;
   if (dim == 3)
-    Az = 0.5 * (Bb[nfx + nfy + i + (int64_t)bx * (j + (int64_t)by * k)] +
-                Bb[nfx + nfy + i + (int64_t)bx * (j + (int64_t)by * (k + 1))]);
+    Az = dscale_down(Bb[nfx + nfy + i + (int64_t)bx * (j + (int64_t)by * k)] +
+                       Bb[nfx + nfy + i + (int64_t)bx * (j + (int64_t)by * (k + 1))],
+                     1);
   else
-    Az = 0.5 * (Bb[nfx + nfy + c] + Bb[nfx + nfy + c]);
-  const double r = fmax(Ub[c], smallr);
-  const double vx = Ub[2 * ncell + c] / r, vy = Ub[3 * ncell + c] / r, vz = Ub[4 * ncell + c] / r;
-  const double eken = 0.5 * (vx * vx + vy * vy + vz * vz);
-  const double emag = 0.5 * (Ax * Ax + Ay * Ay + Az * Az);
-  const double eint = (Ub[ncell + c] - emag) / r - eken;
-  const double p = fmax((gamma0 - 1.0) * r * eint, r * smallp);
-  const double b2 = Ax * Ax + Ay * Ay + Az * Az;
-  const double c2 = gamma0 * p / r;
-  const double d2 = 0.5 * (b2 / r + c2);
-  const double cfx = sqrt(d2 + sqrt(d2 * d2 - c2 * Ax * Ax / r)) + fabs(vx);
-  const double cfy = sqrt(d2 + sqrt(d2 * d2 - c2 * Ay * Ay / r)) + fabs(vy);
-  const double cfz = dim == 3 ? sqrt(d2 + sqrt(d2 * d2 - c2 * Az * Az / r)) + fabs(vz) : 0.0;
-  return cfl_inv_dt_fp64(dim, cfx, cfy, cfz, dx, Ub[c], src);
+    Az = Bb[nfx + nfy + c];
+  const double u[5] = {Ub[c], Ub[ncell + c], Ub[2 * ncell + c], Ub[3 * ncell + c], Ub[4 * ncell + c]};
+  return cell_inv_dt_fp64(u, Ax, Ay, Az, dim, dx, gamma0, smallr, smallp, src);
 }
 
 // FP32 estimate of cfl_inv_dt_fp64 for the mixed path. The gravity factor is evaluated as
@@ -146,6 +161,7 @@ struct Phys
   R   smallc;
   R   smallp;
   R   slope_type;
+  R   entho; // 1 / (gamma0 - 1); FP64 path only
   int riemann;
 };
 
@@ -153,7 +169,7 @@ template <typename R>
 __device__ __forceinline__ R
 dsqrt(R x)
 {
-  return sqrt(x);
+  return sqrt64(x);
 }
 template <>
 __device__ __forceinline__ float
@@ -166,7 +182,7 @@ template <typename R>
 __device__ __forceinline__ R
 rmax(R a, R b)
 {
-  return fmax(a, b);
+  return dmax(a, b);
 }
 template <>
 __device__ __forceinline__ float
@@ -178,7 +194,7 @@ template <typename R>
 __device__ __forceinline__ R
 rmin(R a, R b)
 {
-  return fmin(a, b);
+  return dmin(a, b);
 }
 template <>
 __device__ __forceinline__ float
@@ -211,41 +227,78 @@ rcopysign<float>(float a, float b)
   return copysignf(a, b);
 }
 
-// Divisions that share a divisor. FP64 keeps the reference's x / y (bit-exact parity); the FP32
-// path multiplies by one reciprocal inv = recip(y) computed for all of them (unused, and removed,
-// on the FP64 path).
+// Divisions that share a divisor. FP64 gives the reference's x / y (bit-exact parity) on the integer pipe, with
+// the divisor's reciprocal computed once; the FP32 path multiplies by one reciprocal inv = recip(y).
 template <typename R>
-__device__ __forceinline__ R
+__device__ __forceinline__ auto
 recip(R y)
 {
-  return R(1) / y;
+  if constexpr (std::is_same<R, double>::value)
+    return rcp64(y);
+  else
+    return R(1) / y;
 }
-template <typename R>
+template <typename R, typename I>
 __device__ __forceinline__ R
-qdiv(R x, R y, R inv)
-{
-  (void)inv;
-  return x / y;
-}
-template <>
-__device__ __forceinline__ float
-qdiv<float>(float x, float y, float inv)
+qdiv(R x, R y, const I & inv)
 {
   (void)y;
-  return x * inv;
+  if constexpr (std::is_same<R, double>::value)
+    return div64(x, inv);
+  else
+    return x * inv;
+}
+// x / y as written
+template <typename R>
+__device__ __forceinline__ R
+rdiv(R x, R y)
+{
+  if constexpr (std::is_same<R, double>::value)
+    return div64(x, y);
+  else
+    return x / y;
 }
 // x / sqrt(r): FP64 as written, FP32 as x * rsqrt(r)
 template <typename R>
 __device__ __forceinline__ R
 div_sqrt(R x, R r)
 {
-  return x / dsqrt<R>(r);
+  return rdiv<R>(x, dsqrt<R>(r));
 }
 template <>
 __device__ __forceinline__ float
 div_sqrt<float>(float x, float r)
 {
   return x * rsqrtf(r);
+}
+// q + 0.5 s and q - 0.5 s (0.5 s is exact, so FP64 takes one fused instruction)
+template <typename R>
+__device__ __forceinline__ R
+plus_half(R q, R s)
+{
+  if constexpr (std::is_same<R, double>::value)
+    return fma(0.5, s, q);
+  else
+    return q + R(0.5) * s;
+}
+template <typename R>
+__device__ __forceinline__ R
+minus_half(R q, R s)
+{
+  if constexpr (std::is_same<R, double>::value)
+    return fma(-0.5, s, q);
+  else
+    return q + R(-0.5) * s;
+}
+// x / 2
+template <typename R>
+__device__ __forceinline__ R
+half_of(R x)
+{
+  if constexpr (std::is_same<R, double>::value)
+    return dscale_down(x, 1);
+  else
+    return R(0.5) * x;
 }
 
 // find_speed_fast<dir> (models/mhd_utils.h:93-122)
@@ -254,7 +307,7 @@ __device__ __forceinline__ R
 speed_fast(const R * q, int dir, const Phys<R> & s)
 {
   const R d = q[ID], p = q[IP], a = q[IA], b = q[IB], c = q[IC];
-  const R id = recip<R>(d);
+  const auto id = recip<R>(d);
   const R b2 = a * a + b * b + c * c;
   const R c2 = qdiv<R>(s.gamma0 * p, d, id);
   const R d2 = R(0.5) * (qdiv<R>(b2, d, id) + c2);
@@ -310,7 +363,7 @@ riemann_hll(R * qL, R * qR, R * flux, const Phys<R> & s)
   const R sr = rmax<R>(rmax<R>(vL, vR) + rmax<R>(cfL, cfR), R(0));
 #pragma unroll
   for (int n = 0; n < 8; ++n)
-    flux[n] = (sr * fL[n] - sl * fR[n] + sr * sl * (uR[n] - uL[n])) / (sr - sl);
+    flux[n] = rdiv<R>(sr * fL[n] - sl * fR[n] + sr * sl * (uR[n] - uL[n]), sr - sl);
 }
 
 // riemann_llf (models/RiemannSolvers_MHD.h:118-153)
@@ -403,7 +456,8 @@ riemann_hllc(const R * qL, const R * qR, R * flux, const Phys<R> & s)
   flux[IW] = flux[ID] > R(0) ? flux[ID] * qL[IW] : flux[ID] * qR[IW];
 }
 
-// riemann_hlld (models/RiemannSolvers_MHD.h:311-551), Miyoshi & Kusano 2005
+// riemann_hlld (models/RiemannSolvers_MHD.h:311-551), Miyoshi & Kusano 2005. The mixed path's; FP64:
+// riemann_hlld_fp64.
 template <typename R>
 __device__ void
 riemann_hlld(R * qL, R * qR, R * flux, const Phys<R> & s)
@@ -456,18 +510,9 @@ riemann_hlld(R * qL, R * qR, R * flux, const Phys<R> & s)
   const R vdotbstarl = ustar * a + vstarl * bstarl + wstarl * cstarl;
   const R etotstarl =
     qdiv<R>((sl - ul) * etotl - ptotl * ul + ptotstar * ustar + a * (vdotbl - vdotbstarl), sl - ustar, isl);
-  R sqrrstarl, calfvenl;
-  if constexpr (std::is_same<R, float>::value)
-  {
-    const float rs = rsqrtf(rstarl);
-    sqrrstarl = rstarl * rs;
-    calfvenl = rabs<R>(a) * rs;
-  }
-  else
-  {
-    sqrrstarl = dsqrt<R>(rstarl);
-    calfvenl = rabs<R>(a) / sqrrstarl;
-  }
+  const R rsl = rsqrtf(rstarl);
+  const R sqrrstarl = rstarl * rsl;
+  const R calfvenl = rabs<R>(a) * rsl;
   const R sal = ustar - calfvenl;
 
   const R isr = recip<R>(sr - ustar);
@@ -490,18 +535,9 @@ riemann_hlld(R * qL, R * qR, R * flux, const Phys<R> & s)
   const R vdotbstarr = ustar * a + vstarr * bstarr + wstarr * cstarr;
   const R etotstarr =
     qdiv<R>((sr - ur) * etotr - ptotr * ur + ptotstar * ustar + a * (vdotbr - vdotbstarr), sr - ustar, isr);
-  R sqrrstarr, calfvenr;
-  if constexpr (std::is_same<R, float>::value)
-  {
-    const float rs = rsqrtf(rstarr);
-    sqrrstarr = rstarr * rs;
-    calfvenr = rabs<R>(a) * rs;
-  }
-  else
-  {
-    sqrrstarr = dsqrt<R>(rstarr);
-    calfvenr = rabs<R>(a) / sqrrstarr;
-  }
+  const R rsr = rsqrtf(rstarr);
+  const R sqrrstarr = rstarr * rsr;
+  const R calfvenr = rabs<R>(a) * rsr;
   const R sar = ustar + calfvenr;
 
   const R isq = recip<R>(sqrrstarl + sqrrstarr);
@@ -566,7 +602,12 @@ __device__ __forceinline__ void
 riemann_mhd(R * qL, R * qR, R * flux, const Phys<R> & s)
 {
   if (s.riemann == RS_HLLD)
-    riemann_hlld(qL, qR, flux, s);
+  {
+    if constexpr (std::is_same<R, double>::value)
+      riemann_hlld_fp64(qL, qR, flux, s.gamma0, s.entho);
+    else
+      riemann_hlld(qL, qR, flux, s);
+  }
   else if (s.riemann == RS_HLL)
     riemann_hll(qL, qR, flux, s);
   else if (s.riemann == RS_LLF)
@@ -629,7 +670,8 @@ enum : int
 };
 
 // compute_emf<dir> + mag_riemann2d_hlld (models/RiemannSolvers_MHD.h:629-869, 890-1097).
-// qe[ERT..ELB] are the reconstructed edge states; emf_dir 0 (EMFX), 1 (EMFY), 2 (EMFZ).
+// qe[ERT..ELB] are the reconstructed edge states; emf_dir 0 (EMFX), 1 (EMFY), 2 (EMFZ). The mixed path's; FP64:
+// edge_emf_fp64.
 template <typename R, int EMF_DIR>
 __device__ R
 edge_emf(const R (*qe)[8], const Phys<R> & s)
@@ -665,7 +707,7 @@ edge_emf(const R (*qe)[8], const Phys<R> & s)
 
   // find_speed_fast<IX>/<IY> for the 4 states (models/mhd_utils.h:93-122)
   auto fast = [&](R d, R p, R a, R b, R c, R bn) {
-    const R id = recip<R>(d);
+    const auto id = recip<R>(d);
     const R b2 = a * a + b * b + c * c;
     const R c2 = qdiv<R>(s.gamma0 * p, d, id);
     const R d2 = R(0.5) * (qdiv<R>(b2, d, id) + c2);
@@ -801,6 +843,8 @@ template <typename R>
 __device__ __forceinline__ R
 slope1(R q, R qp, R qm, R slope_type)
 {
+  if constexpr (std::is_same<R, double>::value)
+    return slope1_fp64(q, qp, qm, slope_type);
   R dq = 0;
   if (slope_type == R(1) || slope_type == R(2))
   {

@@ -7,13 +7,20 @@
 
 namespace gmhd
 {
-using F64_3D_844 = Cfg<double, 3, 8, 4, 4, 256, true>;
-using F64_3D_444 = Cfg<double, 3, 4, 4, 4, 64, true>;
+// Threads per tile: 128^3 Orszag-Tang took 18.7 / 17.6 / 17.6 ms with 256 / 384 / 512 threads on the 8x4x4 tile
+// (one CTA per SM either way, by its shared memory), a blast at rest 21.2 / 20.4 / 18.7 ms; blocks of 12^3 (4x4x4
+// tiles) 12.2 ms with 64 threads, 8.2 with 128. The wide variants (_W) are for a launch of so few tiles that each SM
+// holds one or two: 2D 128^2 in 8x8 tiles 131 us with 64 threads, 94 with 128; 16^3 cells in 4x4x4 tiles 156 us with
+// 128 threads, 119 with 256.
+using F64_3D_844 = Cfg<double, 3, 8, 4, 4, 512, true>;
+using F64_3D_444 = Cfg<double, 3, 4, 4, 4, 128, true>;
+using F64_3D_444_W = Cfg<double, 3, 4, 4, 4, 256, true>;
 using F64_2D_16 = Cfg<double, 2, 16, 16, 1, 256, true>;
 using F64_2D_8 = Cfg<double, 2, 8, 8, 1, 64, true>;
+using F64_2D_8_W = Cfg<double, 2, 8, 8, 1, 128, true>;
 using F64_2D_4 = Cfg<double, 2, 4, 4, 1, 32, true>;
-using F64_3D_844_AMR = Cfg<double, 3, 8, 4, 4, 256, true, true>;
-using F64_3D_444_AMR = Cfg<double, 3, 4, 4, 4, 64, true, true>;
+using F64_3D_844_AMR = Cfg<double, 3, 8, 4, 4, 512, true, true>;
+using F64_3D_444_AMR = Cfg<double, 3, 4, 4, 4, 128, true, true>;
 using F64_2D_16_AMR = Cfg<double, 2, 16, 16, 1, 256, true, true>;
 using F64_2D_8_AMR = Cfg<double, 2, 8, 8, 1, 64, true, true>;
 using F64_2D_4_AMR = Cfg<double, 2, 4, 4, 1, 32, true, true>;
@@ -24,14 +31,21 @@ launch_step_fp64_cfg(const StepArgs & a, int dim, cudaStream_t stream)
 {
   int       cand[3];
   const int x = pick_tile(cand, tile_candidates_fp64(dim, a.bx, a.by, a.bz, false, cand), a.tile);
+  const int t = dim == 3 ? 4 : x;
+  const long long tiles =
+    x <= 0 ? 0 : (a.tile_list ? (long long)a.n_list : (long long)a.n_owned * (a.bx / t) * (a.by / t) * (dim == 3 ? a.bz / t : 1));
   if (dim == 3)
   {
     if (x == 8)
       return launch_fused<std::conditional_t<AMR, F64_3D_844_AMR, F64_3D_844>>(a, stream);
+    if (!AMR && tiles <= kSMs)
+      return launch_fused<F64_3D_444_W>(a, stream);
     return launch_fused<std::conditional_t<AMR, F64_3D_444_AMR, F64_3D_444>>(a, stream);
   }
   if (x == 16)
     return launch_fused<std::conditional_t<AMR, F64_2D_16_AMR, F64_2D_16>>(a, stream);
+  if (x == 8 && !AMR && tiles <= 2 * kSMs)
+    return launch_fused<F64_2D_8_W>(a, stream);
   if (x == 8)
     return launch_fused<std::conditional_t<AMR, F64_2D_8_AMR, F64_2D_8>>(a, stream);
   return launch_fused<std::conditional_t<AMR, F64_2D_4_AMR, F64_2D_4>>(a, stream);
@@ -82,11 +96,26 @@ tile_shape_fp64(int dim, int bx, int by, int bz, bool visc, int tile, int * t)
 }
 
 int
+default_tile_fp64(int dim, int bx, int by, int bz, int n_owned)
+{
+  // (FP64 results do not depend on the tile.) 2D: 64 tiles of 16x16 took 154 us, as 8x8 tiles 94 us; 128 tiles 153
+  // against 174. 3D: 32 tiles of 8x4x4 took 175 us, as 4x4x4 tiles 119 us; 96 tiles 174 against 222.
+  const long long half = kSMs / 2;
+  if (dim == 2 && bx % 16 == 0 && by % 16 == 0 && (long long)n_owned * (bx / 16) * (by / 16) <= half)
+    return 8;
+  if (dim == 3 && bx % 8 == 0 && by % 4 == 0 && bz % 4 == 0 && (long long)n_owned * (bx / 8) * (by / 4) * (bz / 4) <= half)
+    return 4;
+  return 0;
+}
+
+int
 prepare_fp64()
 {
   int rc = 0;
   rc = rc ? rc : prepare_fused<F64_3D_844>();
   rc = rc ? rc : prepare_fused<F64_3D_444>();
+  rc = rc ? rc : prepare_fused<F64_3D_444_W>();
+  rc = rc ? rc : prepare_fused<F64_2D_8_W>();
   rc = rc ? rc : prepare_fused<F64_2D_16>();
   rc = rc ? rc : prepare_fused<F64_2D_8>();
   rc = rc ? rc : prepare_fused<F64_2D_4>();

@@ -10,6 +10,7 @@
 #define __host__
 #define __forceinline__ inline
 #define __restrict__
+#include <cstdlib>
 
 static inline long long
 __double_as_longlong(double x)
@@ -83,4 +84,15 @@ static inline float
 rsqrtf(float x)
 {
   return 1.0f / sqrtf(x);
+}
+// the GPU's reciprocal approximations are off by up to this many units in the last place
+static int      host_seed_units = 0;
+static unsigned host_seed_count = 0;
+static inline float
+host_seed(float x)
+{
+  if (!host_seed_units)
+    return x;
+  const int k = (int)(++host_seed_count % (unsigned)(2 * host_seed_units + 1)) - host_seed_units;
+  return __uint_as_float(__float_as_uint(x) + (unsigned)k);
 }

@@ -18,3 +18,17 @@ def test_cfl_screen_bounds(tmp_path):
     """lo <= FP64 value <= hi for every state, tight for most: the screen never drops the maximum."""
     bad, n, tight = map(int, _run(tmp_path, "cfl_bounds_check"))
     assert bad == 0 and n == 320000 and tight > n // 2
+
+
+def test_fp64_on_the_integer_pipe(tmp_path):
+    """Division, square root, min, max, comparisons and power-of-two scalings equal the CPU's FP64 bit for bit, with
+    seeds off by as much as the GPU's approximations may be."""
+    bad, n = map(int, _run(tmp_path, "fp64_int_check", "100000"))
+    assert bad == 0 and n > 6_000_000
+
+
+def test_exact_solvers_match_the_oracle(tmp_path):
+    """Slopes, HLLD fluxes and edge EMFs of the exact path equal the oracle's: independent states, states equal to
+    within 1e-1 .. 0, low beta, supersonic, unmagnetised, degenerate wave fans, NaN."""
+    bad, n = map(int, _run(tmp_path, "exact_solvers_check", "20000"))
+    assert bad == 0 and n == 7_000_000
