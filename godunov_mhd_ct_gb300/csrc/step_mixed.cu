@@ -7,12 +7,12 @@
 namespace gmhd
 {
 using MX_3D_888 = Cfg<float, 3, 8, 8, 8, 512, false>;
-using MX_3D_444 = Cfg<float, 3, 4, 4, 4, 64, false>;
+using MX_3D_444 = Cfg<float, 3, 4, 4, 4, 96, false>;
 using MX_2D_16 = Cfg<float, 2, 16, 16, 1, 256, false>;
 using MX_2D_8 = Cfg<float, 2, 8, 8, 1, 64, false>;
 using MX_2D_4 = Cfg<float, 2, 4, 4, 1, 32, false>;
 using MX_3D_888_AMR = Cfg<float, 3, 8, 8, 8, 512, false, true>;
-using MX_3D_444_AMR = Cfg<float, 3, 4, 4, 4, 64, false, true>;
+using MX_3D_444_AMR = Cfg<float, 3, 4, 4, 4, 96, false, true>;
 using MX_2D_16_AMR = Cfg<float, 2, 16, 16, 1, 256, false, true>;
 using MX_2D_8_AMR = Cfg<float, 2, 8, 8, 1, 64, false, true>;
 using MX_2D_4_AMR = Cfg<float, 2, 4, 4, 1, 32, false, true>;

@@ -8,12 +8,12 @@
 namespace gmhd
 {
 using VMX_3D_884 = Cfg<float, 3, 8, 8, 4, 256, false, false, true>;
-using VMX_3D_444 = Cfg<float, 3, 4, 4, 4, 64, false, false, true>;
+using VMX_3D_444 = Cfg<float, 3, 4, 4, 4, 96, false, false, true>;
 using VMX_2D_16 = Cfg<float, 2, 16, 16, 1, 256, false, false, true>;
 using VMX_2D_8 = Cfg<float, 2, 8, 8, 1, 64, false, false, true>;
 using VMX_2D_4 = Cfg<float, 2, 4, 4, 1, 32, false, false, true>;
 using VMX_3D_884_AMR = Cfg<float, 3, 8, 8, 4, 256, false, true, true>;
-using VMX_3D_444_AMR = Cfg<float, 3, 4, 4, 4, 64, false, true, true>;
+using VMX_3D_444_AMR = Cfg<float, 3, 4, 4, 4, 96, false, true, true>;
 using VMX_2D_16_AMR = Cfg<float, 2, 16, 16, 1, 256, false, true, true>;
 using VMX_2D_8_AMR = Cfg<float, 2, 8, 8, 1, 64, false, true, true>;
 using VMX_2D_4_AMR = Cfg<float, 2, 4, 4, 1, 32, false, true, true>;
