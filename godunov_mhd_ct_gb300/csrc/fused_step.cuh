@@ -2090,63 +2090,56 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
   // of them in shared memory for the CFL of the updated cells. The face loads of this phase and the
   // conservative state of phase 7 are issued together, before either is used.
   double upre[C::CPT][C::NFV];
+  const double * Mx = emfd;
+  const double * My = emfd + (DIM == 3 ? C::NM : 0);
+  const double * Mz = emfd + (DIM == 3 ? 2 * C::NM : 0);
+  const bool     ex = (x0 + TX == bx), ey = (y0 + TY == by), ez = (z0 + TZ == bz);
+  double *       B2blk = a.B2 + (int64_t)blk * a.nface;
+  const double * Bblk = a.B + (int64_t)blk * a.nface;
+  // block-local face index of shared-memory face item n
+  auto face_g = [&](int n) -> int64_t {
+    if (n < C::NB2X)
+    {
+      const int i = n % (TX + 1), j = (n / (TX + 1)) % TY, k = n / ((TX + 1) * TY);
+      return (x0 + i) + (int64_t)(bx + 1) * ((y0 + j) + (int64_t)by * (z0 + k));
+    }
+    if (n < C::NB2X + C::NB2Y)
+    {
+      const int nn = n - C::NB2X;
+      const int i = nn % TX, j = (nn / TX) % (TY + 1), k = nn / (TX * (TY + 1));
+      return a.nfx + (x0 + i) + (int64_t)bx * ((y0 + j) + (int64_t)(by + 1) * (z0 + k));
+    }
+    const int nn = n - C::NB2X - C::NB2Y;
+    const int i = nn % TX, j = (nn / TX) % TY, k = nn / (TX * TY);
+    return a.nfx + a.nfy + (x0 + i) + (int64_t)bx * ((y0 + j) + (int64_t)by * (z0 + k));
+  };
+  constexpr int ITB = (C::NB2 + NT - 1) / NT;
+  double        bold[ITB];
+#pragma unroll
+  for (int it = 0; it < ITB; ++it)
   {
-    const double * Mx = emfd;
-    const double * My = emfd + (DIM == 3 ? C::NM : 0);
-    const double * Mz = emfd + (DIM == 3 ? 2 * C::NM : 0);
-    const bool     ex = (x0 + TX == bx), ey = (y0 + TY == by), ez = (z0 + TZ == bz);
-    double *       B2blk = a.B2 + (int64_t)blk * a.nface;
-    const double * Bblk = a.B + (int64_t)blk * a.nface;
-    // block-local face index of shared-memory face item n
-    auto face_g = [&](int n) -> int64_t {
-      if (n < C::NB2X)
-      {
-        const int i = n % (TX + 1), j = (n / (TX + 1)) % TY, k = n / ((TX + 1) * TY);
-        return (x0 + i) + (int64_t)(bx + 1) * ((y0 + j) + (int64_t)by * (z0 + k));
-      }
-      if (n < C::NB2X + C::NB2Y)
-      {
-        const int nn = n - C::NB2X;
-        const int i = nn % TX, j = (nn / TX) % (TY + 1), k = nn / (TX * (TY + 1));
-        return a.nfx + (x0 + i) + (int64_t)bx * ((y0 + j) + (int64_t)(by + 1) * (z0 + k));
-      }
-      const int nn = n - C::NB2X - C::NB2Y;
-      const int i = nn % TX, j = (nn / TX) % TY, k = nn / (TX * TY);
-      return a.nfx + a.nfy + (x0 + i) + (int64_t)bx * ((y0 + j) + (int64_t)by * (z0 + k));
-    };
-    constexpr int ITB = (C::NB2 + NT - 1) / NT;
-    double        bold[ITB];
+    const int n = tid + it * NT;
+    bold[it] = n < C::NB2 ? Bblk[face_g(n)] : 0.0;
+  }
 #pragma unroll
-    for (int it = 0; it < ITB; ++it)
+  for (int c = 0; c < C::CPT; ++c)
+  {
+    const int n = tid + c * NT;
+#pragma unroll
+    for (int v = 0; v < C::NFV; ++v)
+      upre[c][v] = 0.0;
+    if (n < C::NCELL)
     {
-      const int n = tid + it * NT;
-      bold[it] = n < C::NB2 ? Bblk[face_g(n)] : 0.0;
-    }
+      const int     i = n % TX, j = (n / TX) % TY, k = n / (TX * TY);
+      const int64_t cell = (x0 + i) + (int64_t)bx * ((y0 + j) + (int64_t)by * (z0 + k));
 #pragma unroll
-    for (int c = 0; c < C::CPT; ++c)
-    {
-      const int n = tid + c * NT;
-#pragma unroll
-      for (int v = 0; v < C::NFV; ++v)
-        upre[c][v] = 0.0;
-      if (n < C::NCELL)
-      {
-        const int     i = n % TX, j = (n / TX) % TY, k = n / (TX * TY);
-        const int64_t cell = (x0 + i) + (int64_t)bx * ((y0 + j) + (int64_t)by * (z0 + k));
-#pragma unroll
-        for (int v = 0; v < 5; ++v)
-          upre[c][v] = a.U[((int64_t)blk * 5 + v) * a.ncell + cell];
-        if constexpr (DIM == 2)
-          upre[c][5] = a.B[(int64_t)blk * a.nface + a.nfx + a.nfy + cell];
-      }
+      for (int v = 0; v < 5; ++v)
+        upre[c][v] = a.U[((int64_t)blk * 5 + v) * a.ncell + cell];
+      if constexpr (DIM == 2)
+        upre[c][5] = a.B[(int64_t)blk * a.nface + a.nfx + a.nfy + cell];
     }
-    if constexpr (C::PIPE)
-    {
-      // slopes, predictor and face source are dead: their area receives the next tile's gather while
-      // the loads above are in flight and phases 6-7 run
-      if (has_next)
-        stage_tile(work + gridDim.x, buf ^ 1);
-    }
+  }
+  auto ct_update = [&]() {
 #pragma unroll
     for (int it = 0; it < ITB; ++it)
     {
@@ -2193,22 +2186,18 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
         B2blk[face_g(n)] = bnew;
       b2s[n] = to_r<R>(bnew);
     }
-  }
-  __syncthreads();
+  };
 
   // ---- phase 7: conservative update (ReadFluxesAndConservativeUpdateFunctor.cpp:240-436),
   // write U2 (and 2D Bz), fused CFL of the new state (ComputeDtMHDFunctor.cpp:86-151) ----------
   double my_invdt = 0.0;   // FP64 path
   float  my_invdt_f = 0.0f; // mixed path: FP32 maximum, widened once per CTA
-#pragma unroll
-  for (int c = 0; c < C::CPT; ++c)
-  {
+  auto cell_update = [&](int c, double * u2) {
     const int n = tid + c * NT;
     if (n >= C::NCELL)
-      continue;
+      return;
     const int     i = n % TX, j = (n / TX) % TY, k = n / (TX * TY);
     const int64_t cell = (x0 + i) + (int64_t)bx * ((y0 + j) + (int64_t)by * (z0 + k));
-    double        u2[C::NFV];
 #pragma unroll
     for (int v = 0; v < C::NFV; ++v)
       u2[v] = upre[c][v];
@@ -2393,8 +2382,12 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
         health |= HEALTH_NONFINITE;
     }
 
-    if (a.invdt_out)
+  };
+  auto cell_cfl = [&](int c, const double * u2) {
+    const int n = tid + c * NT;
+    if (n < C::NCELL)
     {
+      const int i = n % TX, j = (n / TX) % TY, k = n / (TX * TY);
       const R Axl = b2s[i + (TX + 1) * (j + TY * k)], Axr = b2s[i + 1 + (TX + 1) * (j + TY * k)];
       const R Ayl = b2s[C::NB2X + i + TX * (j + (TY + 1) * k)], Ayr = b2s[C::NB2X + i + TX * (j + 1 + (TY + 1) * k)];
       [[maybe_unused]] double val = 0.0; // FP64 path
@@ -2438,6 +2431,56 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
       }
       if constexpr (C::EXACT)
         my_invdt = fmax(my_invdt, val);
+    }
+  };
+  if constexpr (C::PIPE && !C::AMR)
+  {
+    // Slopes, predictor and face source are dead: their area receives the next tile's gather. Issuing it is address
+    // arithmetic (9 % of the kernel's instructions), the updates keep the FP64 pipe busy (5 to 10 FP64 additions a face
+    // and a cell, at 16 cycles of the SM's pipe per warp): half the warps begin with one, half with the other. 256^3:
+    // 6.65 -> 6.44 ms a step, 128^3 with viscosity 1.36 -> 1.33. (Coarse/fine variants spill at this; they keep the
+    // order below.)
+    double u2[C::CPT][C::NFV];
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part)
+    {
+      if (((tid >> 5) & 1) == part)
+      {
+        if (has_next)
+          stage_tile(work + gridDim.x, buf ^ 1);
+      }
+      else
+      {
+        ct_update();
+#pragma unroll
+        for (int c = 0; c < C::CPT; ++c)
+          cell_update(c, u2[c]);
+      }
+    }
+    if (a.invdt_out)
+    {
+      __syncthreads();
+#pragma unroll
+      for (int c = 0; c < C::CPT; ++c)
+        cell_cfl(c, u2[c]);
+    }
+  }
+  else
+  {
+    if constexpr (C::PIPE)
+    {
+      if (has_next)
+        stage_tile(work + gridDim.x, buf ^ 1);
+    }
+    ct_update();
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < C::CPT; ++c)
+    {
+      double u2[C::NFV];
+      cell_update(c, u2);
+      if (a.invdt_out)
+        cell_cfl(c, u2);
     }
   }
 
