@@ -200,6 +200,12 @@ struct Cfg
   static constexpr int NCELL = TX * TY * TZ;
   static constexpr int CPT = (NCELL + NT - 1) / NT;
 
+  // rounding variant of the mixed HLLD (riemann_hlld_f32) in direction d
+  __host__ __device__ static constexpr int hlld_fuse(int d)
+  {
+    return !(DIM == 2 && TX == 16) ? HLLD_PLAIN : (AMR && !VISC && d == 0 ? HLLD_FUSE_LR : HLLD_FUSE_R);
+  }
+
   __device__ static int qi(int i, int j, int k) { return (i + 2) + QX * ((j + 2) + QY * (k + 2 * D3)); }
   __device__ static int fxi(int i, int j, int k) { return (i + 2) + (TX + 5) * ((j + 2) + QY * (k + 2 * D3)); }
   __device__ static int fyi(int i, int j, int k) { return (i + 2) + QX * ((j + 2) + (TY + 5) * (k + 2 * D3)); }
@@ -804,7 +810,8 @@ edge_pass(const TileView<C> & t, int tid)
     const int i = m % NX, j = (m / NX) % NY, k = m / (NX * NY);
     R         qe[4][8];
     edge_states<C, CD>(t, i, j, k, qe);
-    store_emf<C, CD>(t, i, j, k, edge_emf<R, CD>(qe, t.ph) * t.dtdx);
+    const R val = edge_emf<R, CD, C::DIM>(qe, t.ph) * t.dtdx;
+    store_emf<C, CD>(t, i, j, k, val);
   }
 }
 
@@ -841,10 +848,12 @@ edge_pass_fp64(const TileView<C> & t, int tid)
         v[q] = st[q][iv];
         c[q] = st[q][ic];
       }
-      a0 = qe[ERT][ia] + qe[ELT][ia];
-      a1 = qe[ERB][ia] + qe[ELB][ia];
-      b0 = qe[ERT][ib] + qe[ERB][ib];
-      b1 = qe[ELT][ib] + qe[ELB][ib];
+      // (the mean of two equal values, except By on x edges: see edge_emf_f32)
+      constexpr bool own = C::DIM == 3 && CD == 0;
+      a0 = own ? dscale_down(qe[ERT][ia] + qe[ELT][ia], 1) : qe[ERT][ia];
+      a1 = own ? dscale_down(qe[ERB][ia] + qe[ELB][ia], 1) : qe[ERB][ia];
+      b0 = qe[ERT][ib];
+      b1 = qe[ELT][ib];
     };
     if (C::DIM == 2 || m < C::NEZ)
       states(std::integral_constant<int, 2>{}, m);
@@ -855,9 +864,7 @@ edge_pass_fp64(const TileView<C> & t, int tid)
       else
         states(std::integral_constant<int, 0>{}, m - C::NEZ - C::NEY);
     }
-    const double val = edge_emf_fp64(r, p, u, v, c, dscale_down(a0, 1), dscale_down(a1, 1), dscale_down(b0, 1),
-                                     dscale_down(b1, 1), t.ph.gamma0, t.ph.smallc) *
-                       t.dtdx;
+    const double val = edge_emf_fp64(r, p, u, v, c, a0, a1, b0, b1, t.ph.gamma0, t.ph.smallc) * t.dtdx;
     if (C::DIM == 2 || m < C::NEZ)
       store_emf<C, 2>(t, i, j, k, val);
     else if constexpr (C::DIM == 3)
@@ -910,7 +917,7 @@ flux_pass(const TileView<C> & t, int tid)
       tmp = qL[IA]; qL[IA] = qL[imag]; qL[imag] = tmp;
       tmp = qR[IA]; qR[IA] = qR[imag]; qR[imag] = tmp;
     }
-    riemann_mhd<R>(qL, qR, flux, t.ph);
+    riemann_mhd<R, C::hlld_fuse(D)>(qL, qR, flux, t.ph);
     if constexpr (D != 0)
     {
       R tmp;
