@@ -330,6 +330,8 @@ __global__ void __launch_bounds__(K::NT, 2) column_step_kernel(const StepArgs a)
   __shared__ float        s_tr[3]; // dx, dt/dx, 1/dx (FP32)
   __shared__ float        s_red[NT / 32];
 
+  next_kernel_may_start();
+  wait_for_kernel_before();
   const int tid = threadIdx.x;
   const int bx = a.bx, by = a.by, bz = a.bz;
   const int cols_x = bx / TX, cols_per_block = cols_x * (by / TY);

@@ -579,9 +579,12 @@ fill_outside_faces_kernel(FillArgs a)
 
 // ---- device-side time control of gmhd_advance -----------------------------------------------
 __global__ void
-advance_time_kernel(const unsigned long long * invdt, double cfl, double * t, const double * t_end, double * dt_cur,
-                    double * dt_log, int32_t * counter, int np, int64_t log_cap, int skip_ok)
+advance_time_kernel(const unsigned long long * invdt, unsigned long long * invdt_next, double cfl, double * t,
+                    const double * t_end, double * dt_cur, double * dt_log, int32_t * counter, int np, int64_t log_cap,
+                    int skip_ok)
 {
+  gmhd::next_kernel_may_start();
+  gmhd::wait_for_kernel_before();
   const int n = *counter;
   for (int p = threadIdx.x; p < np; p += blockDim.x)
   {
@@ -604,6 +607,7 @@ advance_time_kernel(const unsigned long long * invdt, double cfl, double * t, co
       dt = -0.0;
     dt_cur[p] = dt;
     t[p] += dt;
+    invdt_next[p] = 0ull; // (CFL maxima of the step to come)
   }
   __syncthreads();
   if (threadIdx.x == 0)
@@ -687,9 +691,9 @@ enqueue_iteration_rk2(gmhd_ctx * ctx, const double * Uc, double * Un, const doub
                       cudaStream_t s, bool has_tend)
 {
   const int np = ctx->n_problems;
-  advance_time_kernel<<<1, 256, 0, s>>>(ctx->d_invdt + (size_t)slot_in * np, ctx->p.cfl, ctx->d_t,
-                                        has_tend ? ctx->d_tend : nullptr, ctx->d_dt, ctx->d_dtlog, ctx->d_counter,
-                                        np, ctx->dtlog_cap, 0);
+  advance_time_kernel<<<1, 256, 0, s>>>(ctx->d_invdt + (size_t)slot_in * np, ctx->d_invdt + (size_t)(1 - slot_in) * np,
+                                        ctx->p.cfl, ctx->d_t, has_tend ? ctx->d_tend : nullptr, ctx->d_dt, ctx->d_dtlog,
+                                        ctx->d_counter, np, ctx->dtlog_cap, 0);
   GMHD_CUDA(cudaGetLastError());
   int rc = enqueue_fill(ctx, const_cast<double *>(Uc), const_cast<double *>(Bc), s);
   if (rc)
@@ -711,25 +715,26 @@ enqueue_iteration_rk2(gmhd_ctx * ctx, const double * Uc, double * Un, const doub
                         ctx->p.precision != GMHD_PRECISION_MIXED);
 }
 
-// one solver iteration of gmhd_advance: time control, outside fill, fused step + CFL
+// one solver iteration of gmhd_advance: time control, outside fill, fused step + CFL. `first`: what precedes it in the
+// stream or graph may be something other than an iteration's last kernel.
 int
 enqueue_iteration(gmhd_ctx * ctx, const double * Uc, double * Un, const double * Bc, double * Bn, int slot_in,
-                  cudaStream_t s, bool has_tend)
+                  cudaStream_t s, bool has_tend, bool first)
 {
   if (ctx->p.time_integrator == GMHD_TIME_RK2_SSP)
     return enqueue_iteration_rk2(ctx, Uc, Un, Bc, Bn, slot_in, s, has_tend);
   const int np = ctx->n_problems;
-  advance_time_kernel<<<1, 256, 0, s>>>(ctx->d_invdt + (size_t)slot_in * np, ctx->p.cfl, ctx->d_t,
-                                        has_tend ? ctx->d_tend : nullptr, ctx->d_dt, ctx->d_dtlog, ctx->d_counter,
-                                        np, ctx->dtlog_cap, 1);
-  GMHD_CUDA(cudaGetLastError());
   unsigned long long * out = ctx->d_invdt + (size_t)(1 - slot_in) * np;
-  GMHD_CUDA(cudaMemsetAsync(out, 0, sizeof(unsigned long long) * np, s));
+  GMHD_CUDA(gmhd::launch_kernel(advance_time_kernel, 1u, 256, 0, s, !first,
+                                (const unsigned long long *)(ctx->d_invdt + (size_t)slot_in * np), out, ctx->p.cfl,
+                                ctx->d_t, (const double *)(has_tend ? ctx->d_tend : nullptr), ctx->d_dt, ctx->d_dtlog,
+                                ctx->d_counter, np, ctx->dtlog_cap, 1));
   int rc = enqueue_fill(ctx, const_cast<double *>(Uc), const_cast<double *>(Bc), s);
   if (rc)
     return rc;
   gmhd::StepArgs a = make_args(ctx, Uc, Un, Bc, Bn);
   a.dt_dev = ctx->d_dt;
+  a.early = 1;
   a.invdt_out = out;
   return launch_step(ctx, a, s);
 }
@@ -1571,8 +1576,8 @@ gmhd_advance(gmhd_ctx * ctx, double * U, double * U2, double * B, double * B2, i
       }
       cudaGraph_t g = nullptr;
       GMHD_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      int rc1 = enqueue_iteration(ctx, U, U2, B, B2, 0, s, has_tend);
-      int rc2 = rc1 ? rc1 : enqueue_iteration(ctx, U2, U, B2, B, 1, s, has_tend);
+      int rc1 = enqueue_iteration(ctx, U, U2, B, B2, 0, s, has_tend, true);
+      int rc2 = rc1 ? rc1 : enqueue_iteration(ctx, U2, U, B2, B, 1, s, has_tend, false);
       cudaError_t ec = cudaStreamEndCapture(s, &g);
       if (rc2)
       {
@@ -1594,7 +1599,8 @@ gmhd_advance(gmhd_ctx * ctx, double * U, double * U2, double * B, double * B2, i
   for (; done < nsteps; ++done)
   {
     const bool even = (done % 2) == 0;
-    rc = even ? enqueue_iteration(ctx, U, U2, B, B2, 0, s, has_tend) : enqueue_iteration(ctx, U2, U, B2, B, 1, s, has_tend);
+    rc = even ? enqueue_iteration(ctx, U, U2, B, B2, 0, s, has_tend, true)
+              : enqueue_iteration(ctx, U2, U, B2, B, 1, s, has_tend, false);
     if (rc)
       return rc;
   }

@@ -10,6 +10,25 @@ namespace gmhd
 
 constexpr int kSMs = 152;
 
+// kernel<<<grid, threads, smem, stream>>>(args...), with `early` as a programmatic dependent launch: the kernel may start
+// before the one ahead of it in the stream has ended, and waits for that itself (wait_for_kernel_before)
+template <class... P>
+cudaError_t
+launch_kernel(void (*kernel)(P...), unsigned grid, int threads, size_t smem, cudaStream_t stream, bool early, P... args)
+{
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Launch the fused step for configuration C. Returns a cudaError_t (0 on success) or -1 when the
 // tile does not divide the block.
 // Resident CTAs of configuration C on the whole device (persistent variants), set by prepare_fused.
@@ -41,8 +60,8 @@ launch_fused(StepArgs a, cudaStream_t stream)
       return -1;
     nblocks = nblocks < resident_ctas<C>() ? nblocks : resident_ctas<C>();
   }
-  fused_step_kernel<C><<<(unsigned)nblocks, C::NT, C::SMEM_BYTES, stream>>>(a);
-  return (int)cudaGetLastError();
+  return (int)launch_kernel(fused_step_kernel<C>, (unsigned)nblocks, C::NT, C::SMEM_BYTES, stream, a.early != 0,
+                            (const StepArgs)a);
 }
 
 // Opt configuration C into its dynamic shared-memory size on the current device and record how

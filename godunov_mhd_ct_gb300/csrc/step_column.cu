@@ -25,8 +25,7 @@ launch_column(const StepArgs & a, cudaStream_t stream)
   if (g_column_ctas <= 0)
     return -1;
   const long long grid = n_work < g_column_ctas ? n_work : g_column_ctas;
-  column_step_kernel<K><<<(unsigned)grid, K::NT, K::SMEM_BYTES, stream>>>(a);
-  return (int)cudaGetLastError();
+  return (int)launch_kernel(column_step_kernel<K>, (unsigned)grid, K::NT, K::SMEM_BYTES, stream, a.early != 0, a);
 }
 
 int
