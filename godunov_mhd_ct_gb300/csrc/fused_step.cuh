@@ -115,7 +115,7 @@ enum : unsigned int
 };
 
 template <typename R_, int DIM_, int TX_, int TY_, int TZ_, int NT_, bool EXACT_, bool AMR_ = false,
-          bool VISC_ = false>
+          bool VISC_ = false, bool R16_ = (DIM_ == 2 && TX_ == 16)>
 struct Cfg
 {
   using R = R_;
@@ -218,10 +218,11 @@ struct Cfg
   static constexpr int NCELL = TX * TY * TZ;
   static constexpr int CPT = (NCELL + NT - 1) / NT;
 
-  // rounding variant of the mixed HLLD (riemann_hlld_f32) in direction d
+  // rounding variant of the mixed HLLD (riemann_hlld_f32) in direction d: the 2D 16x16 tile's (R16), which a smaller tile
+  // that stands in for it takes too
   __host__ __device__ static constexpr int hlld_fuse(int d)
   {
-    return !(DIM == 2 && TX == 16) ? HLLD_PLAIN : (AMR && !VISC && d == 0 ? HLLD_FUSE_LR : HLLD_FUSE_R);
+    return !R16_ ? HLLD_PLAIN : (AMR && !VISC && d == 0 ? HLLD_FUSE_LR : HLLD_FUSE_R);
   }
 
   __device__ static int qi(int i, int j, int k) { return (i + 2) + QX * ((j + 2) + QY * (k + 2 * D3)); }

@@ -11,11 +11,44 @@ using MX_3D_444 = Cfg<float, 3, 4, 4, 4, 96, false>;
 using MX_2D_16 = Cfg<float, 2, 16, 16, 1, 256, false>;
 using MX_2D_8 = Cfg<float, 2, 8, 8, 1, 64, false>;
 using MX_2D_4 = Cfg<float, 2, 4, 4, 1, 32, false>;
+// The same small tiles with four threads a cell, for meshes that leave SMs idle: such a step takes as long as one tile's
+// chain of phases does. 2D 8x8 also with the rounding of the 16x16 tile, in whose place it runs (few_tiles).
+using MX_3D_444_W = Cfg<float, 3, 4, 4, 4, 256, false>;
+using MX_2D_8_W = Cfg<float, 2, 8, 8, 1, 256, false>;
+using MX_2D_8_W16 = Cfg<float, 2, 8, 8, 1, 256, false, false, false, true>;
 using MX_3D_888_AMR = Cfg<float, 3, 8, 8, 8, 512, false, true>;
 using MX_3D_444_AMR = Cfg<float, 3, 4, 4, 4, 96, false, true>;
 using MX_2D_16_AMR = Cfg<float, 2, 16, 16, 1, 256, false, true>;
 using MX_2D_8_AMR = Cfg<float, 2, 8, 8, 1, 64, false, true>;
 using MX_2D_4_AMR = Cfg<float, 2, 4, 4, 1, 32, false, true>;
+
+// tiles of n x n (x n) cells on the mesh, 0 when they do not divide its blocks
+static long long
+tiles_of(const StepArgs & a, int dim, int n)
+{
+  if (a.bx % n || a.by % n || (dim == 3 && a.bz % n))
+    return 0;
+  return (long long)a.n_owned * (a.bx / n) * (a.by / n) * (dim == 3 ? a.bz / n : 1);
+}
+
+// Meshes of at most half as many of their largest tiles as SMs, when no tile was asked for, run as smaller ones: the same
+// results on more SMs. Twenty steps, us: 2D, 1 / 64 / 81 tiles of 16x16 421 / 437 / 590, as 8x8 with 256 threads 350 / 378 /
+// 678. 3D, 8 / 64 / 125 tiles of 8x8x8 863 / 858 / 1395, as 4x4x4 with 96 threads 717 / 769 / 1887 (with 256: 489 for 8).
+static bool
+few_tiles(const StepArgs & a, int dim)
+{
+  const long long n = tiles_of(a, dim, dim == 3 ? 8 : 16);
+  return a.tile == 0 && !a.tile_list && n > 0 && n <= kSMs / 2;
+}
+
+// Where two small tiles or fewer fall to an SM they take 256 threads. Twenty steps, us: 8 / 64 / 216 / 512 tiles of 4x4x4
+// 679 / 682 / 686 / 738 with 96 threads, 428 / 446 / 516 / 832 with 256; 4 / 64 / 256 / 1024 tiles of 8x8 435 / 418 / 436 /
+// 575 with 64 threads, 346 / 319 / 372 / 892 with 256.
+static bool
+wide(const StepArgs & a, int dim)
+{
+  return tiles_of(a, dim, dim == 3 ? 4 : 8) <= 2 * kSMs;
+}
 
 template <bool AMR>
 int
@@ -27,12 +60,18 @@ launch_step_mixed_cfg(const StepArgs & a, int dim, cudaStream_t stream)
   {
     if (x == 16)
       return launch_column(a, stream);
+    if (!AMR && (x == 4 || few_tiles(a, dim)))
+      return wide(a, dim) ? launch_fused<MX_3D_444_W>(a, stream) : launch_fused<MX_3D_444>(a, stream);
     if (x == 8)
       return launch_fused<std::conditional_t<AMR, MX_3D_888_AMR, MX_3D_888>>(a, stream);
     return launch_fused<std::conditional_t<AMR, MX_3D_444_AMR, MX_3D_444>>(a, stream);
   }
+  if (!AMR && few_tiles(a, dim))
+    return launch_fused<MX_2D_8_W16>(a, stream);
   if (x == 16)
     return launch_fused<std::conditional_t<AMR, MX_2D_16_AMR, MX_2D_16>>(a, stream);
+  if (!AMR && x == 8 && wide(a, dim))
+    return launch_fused<MX_2D_8_W>(a, stream);
   if (x == 8)
     return launch_fused<std::conditional_t<AMR, MX_2D_8_AMR, MX_2D_8>>(a, stream);
   return launch_fused<std::conditional_t<AMR, MX_2D_4_AMR, MX_2D_4>>(a, stream);
@@ -97,6 +136,9 @@ prepare_mixed()
   int rc = 0;
   rc = rc ? rc : prepare_fused<MX_3D_888>();
   rc = rc ? rc : prepare_fused<MX_3D_444>();
+  rc = rc ? rc : prepare_fused<MX_3D_444_W>();
+  rc = rc ? rc : prepare_fused<MX_2D_8_W>();
+  rc = rc ? rc : prepare_fused<MX_2D_8_W16>();
   rc = rc ? rc : prepare_fused<MX_2D_16>();
   rc = rc ? rc : prepare_fused<MX_2D_8>();
   rc = rc ? rc : prepare_fused<MX_2D_4>();
