@@ -50,6 +50,21 @@ __int_as_float(int x)
 {
   return __uint_as_float((unsigned)x);
 }
+static inline float
+__fmul_rn(float x, float y)
+{
+  return x * y;
+}
+static inline float
+__fadd_rn(float x, float y)
+{
+  return x + y;
+}
+static inline float
+__fmaf_rn(float x, float y, float z)
+{
+  return fmaf(x, y, z);
+}
 static inline int
 __double2hiint(double x)
 {
