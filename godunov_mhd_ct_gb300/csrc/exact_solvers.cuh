@@ -5,9 +5,9 @@
 // integer pipe (fp64_int.cuh), and so do comparisons, signs, minima and scalings by powers of two; q + 0.5 s is one fused
 // multiply-add (0.5 s is exact). Where the scheme takes the largest of several speeds, FP32 estimates of their
 // differences show which can be the largest: only those are evaluated in FP64 (one of four fast speeds, one of four
-// Alfven speeds a side; all of them, in the scheme's order, where the estimates are unusable). The weights 0 and 1 of the EMF's nine wave-fan regions become a
-// branch on the region.
-// 3D Orszag-Tang 128^3, FP64: 42.4 -> 17.3 ms a step; 2D 128^2: 315 -> 94 us. The FP64 pipe is still what bounds it
+// Alfven speeds a side; all of them, in the scheme's order, where the estimates are unusable). The weights 0 and 1 of
+// the EMF's nine wave-fan regions become a branch on the region.
+// 3D Orszag-Tang 128^3, FP64: 42.3 -> 16.5 ms a step; 2D 128^2: 315 -> 82 us. The FP64 pipe is still what bounds it
 // (69 % busy), now with the scheme's additions and multiplications.
 #pragma once
 
