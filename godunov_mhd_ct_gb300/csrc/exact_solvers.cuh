@@ -7,8 +7,8 @@
 // differences show which can be the largest: only those are evaluated in FP64 (one of four fast speeds, one of four
 // Alfven speeds a side; all of them, in the scheme's order, where the estimates are unusable). The weights 0 and 1 of
 // the EMF's nine wave-fan regions become a branch on the region.
-// 3D Orszag-Tang 128^3, FP64: 42.3 -> 16.5 ms a step; 2D 128^2: 315 -> 82 us. The FP64 pipe is still what bounds it
-// (69 % busy), now with the scheme's additions and multiplications.
+// 3D Orszag-Tang 128^3, FP64: 42.3 -> 15.0 ms a step; 2D 128^2: 315 -> 82 us. The FP64 pipe is still what bounds it
+// (68 % busy at 16.5 ms), now with the scheme's additions and multiplications.
 #pragma once
 
 #include "fp64_int.cuh"

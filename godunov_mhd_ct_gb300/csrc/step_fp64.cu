@@ -12,14 +12,16 @@ namespace gmhd
 // tiles) 12.2 ms with 64 threads, 8.2 with 128. The wide variants (_W) are for a launch of so few tiles that each SM
 // holds one or two: 2D 128^2 in 8x8 tiles 131 us with 64 threads, 94 with 128; 16^3 cells in 4x4x4 tiles 156 us with
 // 128 threads, 119 with 256.
-using F64_3D_844 = Cfg<double, 3, 8, 4, 4, 512, true>;
+// 8x4x4, one CTA an SM: Orszag-Tang 64^3, ms a step: 2.16 with 384 threads, 2.16 with 512, 1.97 with 576, 2.01 with 640,
+// 2.05 with 768; shear layers with coarse/fine faces 18.04, 17.62, 16.25, 16.31, 16.46.
+using F64_3D_844 = Cfg<double, 3, 8, 4, 4, 576, true>;
 using F64_3D_444 = Cfg<double, 3, 4, 4, 4, 128, true>;
 using F64_3D_444_W = Cfg<double, 3, 4, 4, 4, 256, true>;
 using F64_2D_16 = Cfg<double, 2, 16, 16, 1, 256, true>;
 using F64_2D_8 = Cfg<double, 2, 8, 8, 1, 64, true>;
 using F64_2D_8_W = Cfg<double, 2, 8, 8, 1, 128, true>;
 using F64_2D_4 = Cfg<double, 2, 4, 4, 1, 32, true>;
-using F64_3D_844_AMR = Cfg<double, 3, 8, 4, 4, 512, true, true>;
+using F64_3D_844_AMR = Cfg<double, 3, 8, 4, 4, 576, true, true>;
 using F64_3D_444_AMR = Cfg<double, 3, 4, 4, 4, 128, true, true>;
 using F64_2D_16_AMR = Cfg<double, 2, 16, 16, 1, 256, true, true>;
 using F64_2D_8_AMR = Cfg<double, 2, 8, 8, 1, 64, true, true>;
