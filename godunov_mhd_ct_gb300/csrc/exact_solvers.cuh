@@ -74,18 +74,18 @@ f32_rcp(float x)
   asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 #else
-  return 1.0f / x;
+  return host_seed(1.0f / x);
 #endif
 }
 __device__ __forceinline__ float
-f32_sqrt(float x)
+f32_rsqrt(float x)
 {
 #ifdef __CUDA_ARCH__
   float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 #else
-  return sqrtf(x);
+  return host_seed(1.0f / sqrtf(x));
 #endif
 }
 
@@ -97,17 +97,24 @@ f32_of(double x)
 }
 
 // Which of several nearly equal speeds is the largest is decided on differences: the FP64 differences of the states'
-// values (exact, or nearly) go into FP32, where the difference of two speeds is accurate to a few 2^-24 of the sum of
-// the magnitudes it is made of. kTol covers that (each term is within 25 2^-24 = 1.5e-6); kFloor covers the rounding
-// of the FP64 values themselves (within 1e-13 where the discriminant is at least 1e-5 of the squared speed).
-constexpr float kTol = 4e-6f, kFloor = 1e-12f;
+// values (exact, or nearly) go into FP32. The errors below are relative ones in units of u = 2^-24, to first order:
+//   a value or difference cut to FP32 2, a reciprocal of one 4, a reciprocal square root 3 (the approximations are within 2);
+//   C, X, Y, Z 10 each; h and m of a state 13 of m (h is a difference of terms as large as m); a difference dC .. dZ 19 of the
+//   magnitudes wC .. wZ that it is made of, dm and dh 22 of W / 2.
+// The squared speeds are m + s, s = sqrt(disc), so the difference of two is dm + r N with r = 1 / (s0 + sk) and
+// N = (h0 + hk) dh + Ck (dY + dZ) + T0 dC. N is off by 28 W (m0 + mk) + 33 W (Ck + T0) at most, of which both factors are
+// kept (`e`; with the rest of the sum, and what r adds apart from the next term, 53: kTol is 67). r is off by the error of s:
+// disc's is 26 |h| m + 24 disc, so that s's is 13 q + 15, q = |h| m / disc. Next to equal sound and Alfven speeds q is in the
+// hundreds, and it multiplies the whole of r N (kRel, 20 with 13 needed). kFloor covers the rounding of the FP64 values
+// themselves (within 1e-13 of m where disc is at least 1e-5 m^2).
+constexpr float kTol = 4e-6f, kRel = 1.2e-6f, kFloor = 1e-12f;
 
 // Squared fast speeds along two axes of a state: |b|^2/d and c^2 in FP32 (the field's squares divided by d: X and Y
-// along the two axes, Z the third) and the square roots of the two discriminants, written as
-// ((|b|^2/d - c^2)/2)^2 + c^2 b_t^2/d, free of cancellation.
+// along the two axes, Z the third), the square roots of the two discriminants, written as
+// ((|b|^2/d - c^2)/2)^2 + c^2 b_t^2/d, free of cancellation, and q (see above).
 struct FastEst
 {
-  float id, C, X, Y, Z, h, m, sx, sy;
+  float id, C, X, Y, Z, h, m, sx, sy, qx, qy;
 };
 __device__ __forceinline__ bool
 fast_est(float d, float p, float a, float b, float c, float gamma, FastEst & e)
@@ -121,13 +128,16 @@ fast_est(float d, float p, float a, float b, float c, float gamma, FastEst & e)
   e.h = 0.5f * (t - e.C);
   e.m = 0.5f * (t + e.C);
   const float dx = e.h * e.h + e.C * (e.Y + e.Z), dy = e.h * e.h + e.C * (e.X + e.Z);
-  e.sx = f32_sqrt(dx);
-  e.sy = f32_sqrt(dy);
+  const float ix = f32_rsqrt(dx), iy = f32_rsqrt(dy), hm = fabsf(e.h) * e.m;
+  e.sx = dx * ix;
+  e.sy = dy * iy;
+  e.qx = hm * ix * ix;
+  e.qy = hm * iy * iy;
   const float least = 1e-5f * e.m * e.m;
   return e.m > 1e-12f && e.m < 1e12f && dx > least && dy > least;
 }
-// Squared fast speeds of state k less those of state 0 and the bounds of their errors. dd, dp, da, db, dc: the
-// differences of density, pressure and field; a, b, c: the field's values of the two states.
+// Squared fast speeds of state k less those of state 0 and the bounds of their errors (but for the FP64 values' own). dd, dp,
+// da, db, dc: the differences of density, pressure and field; a, b, c: the field's values of the two states.
 struct FastDiff
 {
   float fx, fy, ex, ey;
@@ -142,17 +152,19 @@ fast_diff(const FastEst & o, const FastEst & k, float dd, float dp, float da, fl
   const float dX = k.id * (da * (a0 + ak) - o.X * dd), wX = k.id * (fabsf(da) * (fabsf(a0) + fabsf(ak)) + o.X * ad);
   const float dY = k.id * (db * (b0 + bk) - o.Y * dd), wY = k.id * (fabsf(db) * (fabsf(b0) + fabsf(bk)) + o.Y * ad);
   const float dZ = k.id * (dc * (c0 + ck) - o.Z * dd), wZ = k.id * (fabsf(dc) * (fabsf(c0) + fabsf(ck)) + o.Z * ad);
-  const float W = wC + wX + wY + wZ;
+  const float W = kTol * (wC + wX + wY + wZ);
   const float dt = dX + dY + dZ;
   const float dm = 0.5f * (dt + dC), dh = 0.5f * (dt - dC);
-  const float hh = o.h + k.h, ah = fabsf(o.h) + fabsf(k.h);
+  const float hh = o.h + k.h, mm = o.m + k.m + k.C;
   const float rx = f32_rcp(o.sx + k.sx), ry = f32_rcp(o.sy + k.sy);
   const float Tx = o.Y + o.Z, Ty = o.X + o.Z;
+  const float px = rx * (hh * dh + k.C * (dY + dZ) + Tx * dC);
+  const float py = ry * (hh * dh + k.C * (dX + dZ) + Ty * dC);
   FastDiff    r;
-  r.fx = dm + rx * (hh * dh + k.C * (dY + dZ) + Tx * dC);
-  r.fy = dm + ry * (hh * dh + k.C * (dX + dZ) + Ty * dC);
-  r.ex = W * (1.0f + rx * (ah + k.C + Tx));
-  r.ey = W * (1.0f + ry * (ah + k.C + Ty));
+  r.fx = dm + px;
+  r.fy = dm + py;
+  r.ex = W * (1.0f + rx * (mm + Tx)) + kRel * (o.qx + k.qx) * fabsf(px);
+  r.ey = W * (1.0f + ry * (mm + Ty)) + kRel * (o.qy + k.qy) * fabsf(py);
   return r;
 }
 
@@ -204,7 +216,7 @@ riemann_hlld_fp64(double * qL, double * qR, double * flux, double gamma, double 
     {
       const FastDiff f =
         fast_diff(el, er, f32_of(rr - rl), f32_of(pr - pl), 0.0f, f32_of(br - bl), f32_of(cr - cl), fa, fa, fbl, fbr, fcl, fcr, gf);
-      const float tol = kTol * f.ex + kFloor * (el.m + er.m);
+      const float tol = f.ex + kFloor * (el.m + er.m);
       left = f.fx <= tol;
       right = f.fx >= -tol;
       // the same state on both sides
@@ -387,8 +399,8 @@ edge_emf_fp64(const double * r, const double * p, const double * u, const double
                                    f32_of(c[k] - c[0]), fa0, ak_f, fb0, bk_f, cf[0], cf[k], gf);
       fx[k] = f.fx;
       fy[k] = f.fy;
-      tx[k] = kTol * f.ex + kFloor * e.m;
-      ty[k] = kTol * f.ey + kFloor * e.m;
+      tx[k] = f.ex + kFloor * e.m;
+      ty[k] = f.ey + kFloor * e.m;
     }
     if (ok)
     {

@@ -106,7 +106,7 @@ static unsigned host_seed_count = 0;
 static inline float
 host_seed(float x)
 {
-  if (!host_seed_units)
+  if (!host_seed_units || !(fabsf(x) > 1.2e-38f && fabsf(x) < 3e38f))
     return x;
   const int k = (int)(++host_seed_count % (unsigned)(2 * host_seed_units + 1)) - host_seed_units;
   return __uint_as_float(__float_as_uint(x) + (unsigned)k);

@@ -1,0 +1,125 @@
+// The FP32 screens of the exact path's speeds (csrc/exact_solvers.cuh) where their margins are thinnest, against the
+// oracle's formulas: equal values (NaN for NaN, zeros of either sign). Arguments: family of states, their number, and by how
+// many units in the last place the FP32 approximations are off. Prints mismatches, comparisons.
+#include <cstdio>
+#include <random>
+#include <string>
+
+#include "host_device_shim.h"
+using std::fma;
+
+#include "../../godunov_mhd_ct_gb300/csrc/exact_solvers.cuh"
+#include "../../oracle/oracle_models.h"
+
+static long bad = 0, n = 0;
+static void
+same(double x, double y, const char * what, long it)
+{
+  ++n;
+  if (!(x == y || (std::isnan(x) && std::isnan(y))) && ++bad <= 5)
+    std::fprintf(stderr, "%s, state %ld: %a not %a\n", what, it, x, y);
+}
+
+// EMFs of the four states qe (RT, LT, RB, LB; fields already shared) along every direction, and the flux of the first two
+static void
+check(const double (*qe)[8], const oracle::Settings & s, long it)
+{
+  for (int dir = 0; dir < 3; ++dir)
+  {
+    const int    iu = dir == 2 ? 2 : (dir == 1 ? 4 : 3), iv = dir == 2 ? 3 : (dir == 1 ? 2 : 4);
+    const int    ia = iu + 3, ib = iv + 3, ic = dir == 2 ? 7 : (dir == 1 ? 6 : 5);
+    const double *RT = qe[0], *LT = qe[1], *RB = qe[2], *LB = qe[3];
+    const double *st[4] = {RT, RB, LT, LB};
+    double       r[4], p[4], u[4], v[4], c[4];
+    for (int k = 0; k < 4; ++k)
+    {
+      r[k] = st[k][0];
+      p[k] = st[k][1];
+      u[k] = st[k][iu];
+      v[k] = st[k][iv];
+      c[k] = st[k][ic];
+    }
+    same(gmhd::edge_emf_fp64(r, p, u, v, c, 0.5 * (RT[ia] + LT[ia]), 0.5 * (RB[ia] + LB[ia]), 0.5 * (RT[ib] + RB[ib]),
+                             0.5 * (LT[ib] + LB[ib]), s.gamma0, s.smallc),
+         oracle::compute_emf(qe, dir, s), "emf", it);
+  }
+  double l1[8], r1[8], l2[8], r2[8], f1[8], f2[8];
+  for (int v = 0; v < 8; ++v)
+  {
+    l1[v] = l2[v] = qe[0][v];
+    r1[v] = r2[v] = qe[1][v];
+  }
+  l1[5] = l2[5] = r1[5] = r2[5];
+  gmhd::riemann_hlld_fp64(l1, r1, f1, s.gamma0, 1.0 / (s.gamma0 - 1.0));
+  oracle::riemann_hlld(l2, r2, f2, s);
+  for (int v = 0; v < 8; ++v)
+    same(f1[v], f2[v], "flux", it);
+}
+
+int
+main(int argc, char ** argv)
+{
+  const std::string                      family = argc > 1 ? argv[1] : "degenerate";
+  const long                             reps = argc > 2 ? std::atol(argv[2]) : 100000;
+  std::mt19937_64                        g(4242);
+  std::uniform_real_distribution<double> U(-1.0, 1.0);
+  host_seed_units = argc > 3 ? std::atoi(argv[3]) : 0;
+  auto       mag = [&](double lo, double hi) { return std::pow(10.0, lo + (hi - lo) * (0.5 + 0.5 * U(g))); };
+  const auto s0 = oracle::make_settings(5.0 / 3.0, 0.5, 2.0, 1e-10, 1e-10, 5);
+
+  if (family == "degenerate")
+  {
+    // the four fast speeds along the field within 1e-9 of one another but for the first (an EMF off by 4e-11 with a
+    // margin that leaves out the error of the discriminant's root)
+    const double r[4] = {0x1.7c7b2770c459ap+1, 0x1.7c7b27a5361cbp+1, 0x1.7c7b27b3bb85ep+1, 0x1.7c7b27970469fp+1};
+    const double p[4] = {0x1.57e33a14f0743p-1, 0x1.57e33a2b348d7p-1, 0x1.57e339f75676cp-1, 0x1.57e33a238ff67p-1};
+    const double u[4] = {-0x1.e584860e4126ep-1, 0x1.92299a18ae8c2p-1, 0x1.664a7c5776298p-1, -0x1.0b8a86ecd4b35p-1};
+    const double v[4] = {0x1.3e62ec79f06c4p-2, -0x1.80ce6142a682p-1, -0x1.3427d63028228p-1, 0x1.113fcbd6a4c22p-1};
+    const double c[4] = {0x1.4ba81078f4feap-9, 0x1.1b499cb75df1p-8, 0x1.1b49abc6093afp-8, 0x1.1b49af1c148fbp-8};
+    const double a[2] = {0x1.0f97dc11ff7a5p+0, 0x1.0f97dbf4a863ep+0}, b = 0x1.842f09b3884fcp-13;
+    double       qe[4][8];
+    const int    at[4] = {0, 2, 1, 3}; // LL, LR, RL, RR: RT, RB, LT, LB
+    for (int k = 0; k < 4; ++k)
+    {
+      const double q[8] = {r[k], p[k], u[k], v[k], 0.0, a[k & 1], b, c[k]};
+      std::copy(q, q + 8, qe[at[k]]);
+    }
+    check(qe, s0, -1);
+  }
+  for (long it = 0; it < reps; ++it)
+  {
+    const auto s = oracle::make_settings(it % 2 ? 5.0 / 3.0 : 1.4, 0.5, 2.0, 1e-10, 1e-10, 5);
+    double base[8], vs, bs, e[4];
+    if (family == "degenerate")
+    {
+      // sound and Alfven speed along one axis nearly equal, a transverse field of 1e-4 to 0.1 of the normal one; three
+      // states alike, one apart (kinds 0 to 3), or two and two (kind 4)
+      const int    axis = it % 3, apart = it / 3 % 8 < 4 ? 0 : it / 3 % 5;
+      const double tf = it % 5 ? mag(-3, -1.5) : mag(-4, -1), rho = mag(-1, 1), near = mag(-10, -5), away = mag(-2, -0.1);
+      vs = mag(-1, 0.5);
+      bs = std::sqrt(rho) * mag(-1, 1);
+      const double detune = it % 7 == 0 ? 0.0 : (it & 1 ? 1 : -1) * (it % 5 ? mag(-3, -2) : tf * mag(-2, 1));
+      base[0] = rho;
+      base[1] = bs * bs / s.gamma0 * (1.0 + detune);
+      for (int d = 0; d < 3; ++d)
+      {
+        base[2 + d] = vs * U(g);
+        base[5 + d] = d == axis ? bs : bs * tf * U(g);
+      }
+      for (int k = 0; k < 4; ++k)
+        e[k] = k == apart || (apart == 4 && k < 2) ? away : near;
+      double qe[4][8];
+      for (int k = 0; k < 4; ++k)
+        for (int w = 0; w < 8; ++w)
+        {
+          // (transverse fields differ by their own size, the rest by a small part of it)
+          const bool   t = w >= 5 && w - 5 != axis;
+          const double x = w >= 2 && w < 5 ? 1.0 : (t ? e[k] : near * mag(-3, 0));
+          qe[k][w] = base[w] + x * (w >= 2 && w < 5 ? vs : std::fabs(base[w])) * U(g);
+        }
+      check(qe, s, it);
+    }
+  }
+  std::printf("%ld %ld\n", bad, n);
+  return 0;
+}

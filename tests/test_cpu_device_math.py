@@ -32,3 +32,11 @@ def test_exact_solvers_match_the_oracle(tmp_path):
     within 1e-1 .. 0, low beta, supersonic, unmagnetised, degenerate wave fans, NaN."""
     bad, n = map(int, _run(tmp_path, "exact_solvers_check", "20000"))
     assert bad == 0 and n == 7_000_000
+
+
+@pytest.mark.parametrize("units", ["0", "1"])
+def test_speed_screens_near_equal_speeds(tmp_path, units):
+    """Fast speeds nearly equal next to equal sound and Alfven speeds, where the discriminant's error is largest, with the
+    FP32 approximations exact and off by one unit in the last place: the largest is the oracle's."""
+    bad, n = map(int, _run(tmp_path, "speed_screen_check", "degenerate", "400000", units))
+    assert bad == 0 and n == 11 * 400_001
