@@ -106,7 +106,9 @@ f32_of(double x)
 // kept (`e`; with the rest of the sum, and what r adds apart from the next term, 53: kTol is 67). r is off by the error of s:
 // disc's is 26 |h| m + 24 disc, so that s's is 13 q + 15, q = |h| m / disc. Next to equal sound and Alfven speeds q is in the
 // hundreds, and it multiplies the whole of r N (kRel, 20 with 13 needed). kFloor covers the rounding of the FP64 values
-// themselves (within 1e-13 of m where disc is at least 1e-5 m^2).
+// themselves (within 1e-13 of m where disc is at least 1e-5 m^2) and what FP32 cuts off: a difference of densities, pressures
+// or fields below 2^-126 = 1.2e-38 counts as zero, which shifts dm + r N by up to 1000 times its share of d or of d m. With both
+// at least 1e-20 that is 2e-15 of m; the upper limits keep the products finite.
 constexpr float kTol = 4e-6f, kRel = 1.2e-6f, kFloor = 1e-12f;
 
 // Squared fast speeds along two axes of a state: |b|^2/d and c^2 in FP32 (the field's squares divided by d: X and Y
@@ -133,8 +135,8 @@ fast_est(float d, float p, float a, float b, float c, float gamma, FastEst & e)
   e.sy = dy * iy;
   e.qx = hm * ix * ix;
   e.qy = hm * iy * iy;
-  const float least = 1e-5f * e.m * e.m;
-  return e.m > 1e-12f && e.m < 1e12f && dx > least && dy > least;
+  const float least = 1e-5f * e.m * e.m, dm = d * e.m;
+  return e.m > 1e-12f && e.m < 1e12f && d > 1e-20f && d < 1e30f && dm > 1e-20f && dm < 1e30f && dx > least && dy > least;
 }
 // Squared fast speeds of state k less those of state 0 and the bounds of their errors (but for the FP64 values' own). dd, dp,
 // da, db, dc: the differences of density, pressure and field; a, b, c: the field's values of the two states.

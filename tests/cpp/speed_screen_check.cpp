@@ -88,7 +88,8 @@ main(int argc, char ** argv)
   }
   for (long it = 0; it < reps; ++it)
   {
-    const auto s = oracle::make_settings(it % 2 ? 5.0 / 3.0 : 1.4, 0.5, 2.0, 1e-10, 1e-10, 5);
+    const double floor = family == "scales" ? 1e-40 : 1e-10;
+    const auto   s = oracle::make_settings(it % 2 ? 5.0 / 3.0 : 1.4, 0.5, 2.0, floor, floor, 5);
     double base[8], vs, bs, e[4];
     if (family == "degenerate")
     {
@@ -117,6 +118,25 @@ main(int argc, char ** argv)
           const double x = w >= 2 && w < 5 ? 1.0 : (t ? e[k] : near * mag(-3, 0));
           qe[k][w] = base[w] + x * (w >= 2 && w < 5 ? vs : std::fabs(base[w])) * U(g);
         }
+      check(qe, s, it);
+    }
+    if (family == "scales")
+    {
+      // densities of 1e-36 to 1e34 at speeds of 1e-4 to 1e4, neighbours within 1e-1 to 1e-14, every fourth with a weak field
+      const double rho = mag(-36, 34), close = mag(-14, -1);
+      vs = mag(-4, 4);
+      bs = std::sqrt(rho) * vs * (it % 4 ? mag(-2, 0.5) : mag(-16, 0));
+      base[0] = rho;
+      base[1] = rho * vs * vs * mag(-1, 1);
+      for (int d = 0; d < 3; ++d)
+      {
+        base[2 + d] = vs * U(g);
+        base[5 + d] = bs * U(g);
+      }
+      double qe[4][8];
+      for (auto & q : qe)
+        for (int w = 0; w < 8; ++w)
+          q[w] = base[w] * (1.0 + close * U(g));
       check(qe, s, it);
     }
   }

@@ -40,3 +40,10 @@ def test_speed_screens_near_equal_speeds(tmp_path, units):
     FP32 approximations exact and off by one unit in the last place: the largest is the oracle's."""
     bad, n = map(int, _run(tmp_path, "speed_screen_check", "degenerate", "400000", units))
     assert bad == 0 and n == 11 * 400_001
+
+
+@pytest.mark.parametrize("units", ["0", "1"])
+def test_speed_screens_at_any_scale(tmp_path, units):
+    """Densities, pressures and squared fields down to the end of the FP32 range and past it, with tiny floors."""
+    bad, n = map(int, _run(tmp_path, "speed_screen_check", "scales", "400000", units))
+    assert bad == 0 and n == 11 * 400_000
