@@ -493,9 +493,12 @@ edge_emf_fp64(const double * r, const double * p, const double * u, const double
   double calf[4];
   {
     float va[4], vb[4], wx[4], wy[4]; // a^2 / |nx|, b^2 / |ny|, v times w
-    bool  ok = true;
+    bool  ok;
     {
       const float fL = f32_rcp(f32_of(dL)), fR = f32_rcp(f32_of(dR)), fB = f32_rcp(f32_of(dB)), fT = f32_rcp(f32_of(dT));
+      // a difference cut to zero below 1.2e-38 is then below 1e-14 of dL .. dT
+      auto held = [](float x) { return fabsf(x) > 1e-24f && fabsf(x) < 1e24f; };
+      ok = held(fL) && held(fR) && held(fB) && held(fT);
 #pragma unroll
       for (int k = 0; k < 4; ++k)
       {
@@ -545,7 +548,8 @@ edge_emf_fp64(const double * r, const double * p, const double * u, const double
         const float e[4] = {0.0f, w0, dv, dv + w1};
         const float t[4] = {fl, kTol * fabsf(w0) + fl, kTol * ev + fl, kTol * (ev + fabsf(w1)) + fl};
         todo = screen4(e, t);
-        todo = fmaxf(v0, v1) > 1e-25f ? todo : 15u;
+        // (products of the fields are off by up to 1e-45 below 1e-38: less than kFloor of a square of 1e-32)
+        todo = fmaxf(v0, v1) > 1e-25f && fmaxf(fabsf(f0), fabsf(f1)) > 1e-16f ? todo : 15u;
       }
       // num / sqrt(rho) grows with num and falls with rho, rounded as well: of two candidates ordered in both only one
       // is evaluated (a uniform state's four differ by roundings of rho and num, if at all)

@@ -47,3 +47,10 @@ def test_speed_screens_at_any_scale(tmp_path, units):
     """Densities, pressures and squared fields down to the end of the FP32 range and past it, with tiny floors."""
     bad, n = map(int, _run(tmp_path, "speed_screen_check", "scales", "400000", units))
     assert bad == 0 and n == 11 * 400_000
+
+
+@pytest.mark.parametrize("units", ["0", "1"])
+def test_alfven_screen_of_weak_fields(tmp_path, units):
+    """Alfven speeds of fields whose squares are near the end of the FP32 range."""
+    bad, n = map(int, _run(tmp_path, "speed_screen_check", "weak", "1000000", units))
+    assert bad == 0 and n == 11 * 1_000_000
