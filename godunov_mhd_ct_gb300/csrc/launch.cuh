@@ -26,7 +26,10 @@ launch_kernel(void (*kernel)(P...), unsigned grid, int threads, size_t smem, cud
   cfg.stream = stream;
   cfg.attrs = &at;
   cfg.numAttrs = early ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess)
+    (void)cudaGetLastError(); // reported here: not left for the next, unrelated check
+  return e;
 }
 
 // Launch the fused step for configuration C. Returns a cudaError_t (0 on success) or -1 when the
