@@ -29,7 +29,7 @@ frsqrt_approx(float x)
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 #else
-  return 1.0f / sqrtf(x);
+  return host_seed(1.0f / sqrtf(x));
 #endif
 }
 
@@ -49,11 +49,13 @@ cut_to_f32(double x, uint32_t & top)
 // gamma - 1 (gm1) to FP32 accuracy.
 //
 // Error model, e = 2^-24: every FP32 input and operation is within 2 e (approximate ones 4 e). The thermal
-// energy and the squared field come from differences, so their error is absolute: at most 32 e times
+// energy and the squared field come from differences, so their error is absolute: at most 15 e times
 // tot = |E| + kinetic + magnetic energy with the face magnitudes in place of their means. The squared fast
-// speed grows with c^2, b_n^2 / rho and b_t^2 / rho at most one for one, so its error is at most
-// delta = (gamma (gamma - 1) + 2) 32 e tot / rho plus its own rounding, which the final factors
-// 1 +- 64 e cover. Cells outside the range where this holds (tiny or huge or non-finite values, or a
+// speed d2 + sqrt(disc) changes by at most twice the change of c^2 or b_n^2 / rho. Its slope in b_t^2 / rho is
+// 1/2 + d2 / (2 sqrt(disc)), up to 160 at the limit of disc below, but sqrt(disc) is at least c b_t / sqrt(rho) and the
+// error of b_t^2 is 2 b_t times that of b_t (2 e of the face magnitudes M), so that it adds 2 e c M / sqrt(rho) at most, less
+// than e (c^2 + M^2 / rho). All of it is within delta = (gamma (gamma - 1) + 2) 32 e tot / rho plus the speed's own rounding,
+// which the final factors 1 +- 64 e cover. Cells outside the range where this holds (tiny or huge or non-finite values, or a
 // discriminant near zero, where the FP64 formula itself may return NaN, which the maximum ignores) give
 // lo = 0, hi = infinity: they are always evaluated.
 __device__ __forceinline__ CflBounds
@@ -72,7 +74,7 @@ cell_inv_dt_bounds(const double * u, const double * f, int dim, float idx, float
 #ifdef __CUDA_ARCH__
   const float ir = __fdividef(1.0f, r);
 #else
-  const float ir = 1.0f / r;
+  const float ir = host_seed(1.0f / r);
 #endif
   const float vx = cut_to_f32(u[2], top) * ir, vy = cut_to_f32(u[3], top) * ir, vz = cut_to_f32(u[4], top) * ir;
   const float ekin = 0.5f * r * (vx * vx + vy * vy + vz * vz);

@@ -85,11 +85,6 @@ __funnelshift_l(unsigned lo, unsigned hi, unsigned s)
 {
   return (unsigned)(((((uint64_t)hi << 32) | lo) << (s & 31)) >> 32);
 }
-static inline uint64_t
-__umul64hi(uint64_t a, uint64_t b)
-{
-  return (uint64_t)(((unsigned __int128)a * b) >> 64);
-}
 static inline unsigned
 __umulhi(unsigned a, unsigned b)
 {
@@ -101,7 +96,10 @@ rsqrtf(float x)
   return 1.0f / sqrtf(x);
 }
 // the GPU's reciprocal approximations are off by up to this many units in the last place
-static int      host_seed_units = 0;
+#ifndef HOST_SEED_UNITS
+#define HOST_SEED_UNITS 0
+#endif
+static int      host_seed_units = HOST_SEED_UNITS;
 static unsigned host_seed_count = 0;
 static inline float
 host_seed(float x)

@@ -7,10 +7,11 @@ import pytest
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
-def _run(tmp_path, name, *args):
+def _run(tmp_path, name, *args, units=0):
     exe = str(tmp_path / name)
     src = os.path.join(HERE, "cpp", name + ".cpp")
-    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fno-strict-aliasing", "-w", src, "-o", exe], check=True)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fno-strict-aliasing", "-w",
+                    f"-DHOST_SEED_UNITS={units}", src, "-o", exe], check=True)
     return subprocess.run([exe, *args], check=True, capture_output=True, text=True).stdout.split()
 
 
@@ -54,3 +55,9 @@ def test_alfven_screen_of_weak_fields(tmp_path, units):
     """Alfven speeds of fields whose squares are near the end of the FP32 range."""
     bad, n = map(int, _run(tmp_path, "speed_screen_check", "weak", "1000000", units))
     assert bad == 0 and n == 11 * 1_000_000
+
+
+def test_cfl_screen_bounds_with_approximate_reciprocals(tmp_path):
+    """As test_cfl_screen_bounds, with reciprocals and reciprocal square roots off by two units in the last place."""
+    bad, n, tight = map(int, _run(tmp_path, "cfl_bounds_check", units=2))
+    assert bad == 0 and n == 320000 and tight > n // 2
