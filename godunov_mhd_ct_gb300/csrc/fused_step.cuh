@@ -218,11 +218,13 @@ struct Cfg
   static constexpr int NCELL = TX * TY * TZ;
   static constexpr int CPT = (NCELL + NT - 1) / NT;
 
-  // rounding variant of the mixed HLLD (riemann_hlld_f32) in direction d: the 2D 16x16 tile's (R16), which a smaller tile
-  // that stands in for it takes too
+  // Rounding of the mixed HLLD (riemann_hlld_f32) on the faces along d: what the compiler once chose for each of these kernels,
+  // kept so that their results stay the same. R16: the 2D 16x16 tile's, which a smaller tile that stands in for it takes too.
   __host__ __device__ static constexpr int hlld_fuse(int d)
   {
-    return !R16_ ? HLLD_PLAIN : (AMR && !VISC && d == 0 ? HLLD_FUSE_LR : HLLD_FUSE_R);
+    if (R16_)
+      return AMR && (VISC || d == 0) ? HLLD_FUSE_LR : HLLD_FUSE_R;
+    return DIM == 3 && TX == 8 && AMR && !VISC ? HLLD_FUSE_R : HLLD_PLAIN;
   }
 
   __device__ static int qi(int i, int j, int k) { return (i + 2) + QX * ((j + 2) + QY * (k + 2 * D3)); }

@@ -459,7 +459,8 @@ riemann_hllc(const R * qL, const R * qR, R * flux, const Phys<R> & s)
 // ---- mixed path: HLLD fluxes and edge EMFs with every FP32 rounding written out -------------------------------
 // Which product of a sum like a b + c d is fused into an FMA is the compiler's choice, and it chose differently from one
 // tile's kernel to another (and from one edit to the next): results of the mixed path then differ in the last FP32
-// bits. The two solvers below name each operation, so that every kernel gives the same bits.
+// bits. The two solvers below name each operation, so that a kernel's bits do not change with the code around them. The edge
+// solver rounds alike in every kernel; HLLD keeps the three forms that the kernels had (below).
 __device__ __forceinline__ float
 fmul_(float a, float b)
 {
@@ -482,8 +483,8 @@ dif2(float a, float b, float c, float d)
   return __fmaf_rn(a, b, -__fmul_rn(c, d));
 }
 
-// The rounding of r (S - u)^2 - a^2 on the left and right side (e): the product fused with the subtraction or not. The
-// 2D meshes of blocks that 16 divides have their own, from the kernel that has always run them.
+// The rounding of r (S - u)^2 - a^2 on the left and right side (e): the product fused with the subtraction or not, as each
+// kernel has always had it (Cfg::hlld_fuse). No form is more accurate than the others by more than an FP32 rounding.
 enum : int
 {
   HLLD_PLAIN = 0,  // neither
