@@ -234,7 +234,7 @@ col_edge(const ColView<K> & t, const ColCtx & c, int i, int j, int p)
   // y edges: the reference swaps the RB and LT states (ComputeEmfAndStoreFunctor.cpp:551-560)
   col_recon_edge<K, D0, D1, LOC_RB>(t, ci(-1, 0), cj(-1, 0), cp(0), c.ph, c.rk2, qe[CD == 1 ? ELT : ERB]);
   col_recon_edge<K, D0, D1, LOC_LT>(t, ci(0, -1), cj(0, -1), cp(-1), c.ph, c.rk2, qe[CD == 1 ? ERB : ELT]);
-  float val = edge_emf<float, CD, 3>(qe, c.ph) * c.dtdx;
+  float val = edge_emf<CD, 3>(qe, c.ph) * c.dtdx;
   const int gi[3] = {c.x0 + i, c.y0 + j, p};
   const int bs[3] = {c.bx, c.by, c.bz};
   const int v0 = gi[D0] == 0 ? -1 : (gi[D0] == bs[D0] ? 1 : 0);

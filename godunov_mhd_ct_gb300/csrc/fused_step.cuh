@@ -831,7 +831,7 @@ edge_pass(const TileView<C> & t, int tid)
     const int i = m % NX, j = (m / NX) % NY, k = m / (NX * NY);
     R         qe[4][8];
     edge_states<C, CD>(t, i, j, k, qe);
-    const R val = edge_emf<R, CD, C::DIM>(qe, t.ph) * t.dtdx;
+    const R val = edge_emf<CD, C::DIM>(qe, t.ph) * t.dtdx;
     store_emf<C, CD>(t, i, j, k, val);
   }
 }

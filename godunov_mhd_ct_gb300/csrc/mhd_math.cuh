@@ -214,19 +214,6 @@ rabs<float>(float a)
 {
   return fabsf(a);
 }
-template <typename R>
-__device__ __forceinline__ R
-rcopysign(R a, R b)
-{
-  return copysign(a, b);
-}
-template <>
-__device__ __forceinline__ float
-rcopysign<float>(float a, float b)
-{
-  return copysignf(a, b);
-}
-
 // Divisions that share a divisor. FP64 gives the reference's x / y (bit-exact parity) on the integer pipe, with
 // the divisor's reciprocal computed once; the FP32 path multiplies by one reciprocal inv = recip(y).
 template <typename R>
@@ -257,19 +244,6 @@ rdiv(R x, R y)
     return div64(x, y);
   else
     return x / y;
-}
-// x / sqrt(r): FP64 as written, FP32 as x * rsqrt(r)
-template <typename R>
-__device__ __forceinline__ R
-div_sqrt(R x, R r)
-{
-  return rdiv<R>(x, dsqrt<R>(r));
-}
-template <>
-__device__ __forceinline__ float
-div_sqrt<float>(float x, float r)
-{
-  return x * rsqrtf(r);
 }
 // q + 0.5 s and q - 0.5 s (0.5 s is exact, so FP64 takes one fused instruction)
 template <typename R>
@@ -741,16 +715,16 @@ edge_emf_f32(const float * r, const float * p, const float * u, const float * v,
 }
 
 // EMF along CD from the reconstructed states qe[ERT..ELB]
-template <typename R, int CD, int DIM>
-__device__ __forceinline__ R
-edge_emf(const R (*qe)[8], const Phys<R> & s)
+template <int CD, int DIM>
+__device__ __forceinline__ float
+edge_emf(const float (*qe)[8], const Phys<float> & s)
 {
   // (u, v) and (a, b) the edge's transverse axes in turn, c along it
   constexpr int  iu = CD == 2 ? IU : (CD == 1 ? IW : IV), iv = CD == 2 ? IV : (CD == 1 ? IU : IW);
   constexpr int  ia = iu + 3, ib = iv + 3, ic = CD == 2 ? IC : (CD == 1 ? IB : IA);
   constexpr bool own = DIM == 3 && CD == 0; // By on x edges: the scheme adds each cell's own slopes to the face's
-  const R *      st[4] = {qe[ERT], qe[ERB], qe[ELT], qe[ELB]};
-  R              r[4], p[4], u[4], v[4], c[4];
+  const float *  st[4] = {qe[ERT], qe[ERB], qe[ELT], qe[ELB]};
+  float          r[4], p[4], u[4], v[4], c[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q)
   {
@@ -760,8 +734,8 @@ edge_emf(const R (*qe)[8], const Phys<R> & s)
     v[q] = st[q][iv];
     c[q] = st[q][ic];
   }
-  const R a0 = own ? half_of<R>(qe[ERT][ia] + qe[ELT][ia]) : qe[ERT][ia];
-  const R a1 = own ? half_of<R>(qe[ERB][ia] + qe[ELB][ia]) : qe[ERB][ia];
+  const float a0 = own ? half_of<float>(qe[ERT][ia] + qe[ELT][ia]) : qe[ERT][ia];
+  const float a1 = own ? half_of<float>(qe[ERB][ia] + qe[ELB][ia]) : qe[ERB][ia];
   return edge_emf_f32(r, p, u, v, c, a0, a1, qe[ERT][ib], qe[ELT][ib], s);
 }
 
