@@ -227,6 +227,9 @@ struct Cfg
     return DIM == 3 && TX == 8 && AMR && !VISC ? HLLD_FUSE_R : HLLD_PLAIN;
   }
 
+  // the same for the gravity half kick of the predictor
+  static constexpr bool KICK_FUSED = R16_ && AMR && VISC;
+
   __device__ static int qi(int i, int j, int k) { return (i + 2) + QX * ((j + 2) + QY * (k + 2 * D3)); }
   __device__ static int fxi(int i, int j, int k) { return (i + 2) + (TX + 5) * ((j + 2) + QY * (k + 2 * D3)); }
   __device__ static int fyi(int i, int j, int k) { return (i + 2) + QX * ((j + 2) + (TY + 5) * (k + 2 * D3)); }
@@ -1882,10 +1885,10 @@ __global__ void __launch_bounds__(C::NT, C::MINB) fused_step_kernel(const StepAr
     if (a.src.gravity)
     {
       const R hdt = (R)dt;
-      ug += (R)a.src.g[0] * R(0.5) * hdt;
-      vg += (R)a.src.g[1] * R(0.5) * hdt;
+      ug = half_kick<R, C::KICK_FUSED>(ug, (R)a.src.g[0], hdt);
+      vg = half_kick<R, C::KICK_FUSED>(vg, (R)a.src.g[1], hdt);
       if constexpr (DIM == 3)
-        wg += (R)a.src.g[2] * R(0.5) * hdt;
+        wg = half_kick<R, C::KICK_FUSED>(wg, (R)a.src.g[2], hdt);
     }
     if constexpr (C::VISC)
     {

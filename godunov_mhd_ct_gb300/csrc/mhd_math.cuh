@@ -457,6 +457,19 @@ dif2(float a, float b, float c, float d)
   return __fmaf_rn(a, b, -__fmul_rn(c, d));
 }
 
+// v + g dt / 2; FP32 with the product fused with the addition or not, as each kernel has always had it (Cfg::KICK_FUSED)
+template <typename R, bool FUSED>
+__device__ __forceinline__ R
+half_kick(R v, R g, R dt)
+{
+  if constexpr (std::is_same<R, double>::value)
+    return v + g * 0.5 * dt;
+  else if constexpr (FUSED)
+    return __fmaf_rn(0.5f * g, dt, v);
+  else
+    return fadd_(v, fmul_(0.5f * g, dt));
+}
+
 // The rounding of r (S - u)^2 - a^2 on the left and right side (e): the product fused with the subtraction or not, as each
 // kernel has always had it (Cfg::hlld_fuse). No form is more accurate than the others by more than an FP32 rounding.
 enum : int

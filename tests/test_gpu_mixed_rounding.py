@@ -1,5 +1,5 @@
 """Every kernel of the mixed step rounds as it always has: SHA-256 digests of one step's U2 and B2, recorded before the edge
-solver and HLLD named their roundings. (The other phases' FP32 contractions are the compiler's: another nvcc may need new
+solver, HLLD and the gravity kick named their roundings. (The other phases' FP32 contractions are the compiler's: another nvcc may need new
 digests.) States come from integer hashes and plain arithmetic only, so that the host's math library has no part in them."""
 import hashlib
 
@@ -55,13 +55,13 @@ def _state(mesh):
     return U, B
 
 
-def digest(dim, block, amr, mu):
+def digest(dim, block, amr, mu, gravity=None, dt=2.0 ** -13):
     mesh = _mesh(dim, block, amr)
-    impl = GodunovImplemGB300(MHDSettings(gamma0=1.4, cfl=0.4, slope_type=2.0, riemann="HLLD", viscosity_mu=mu or None), mesh,
-                              precision="mixed")
+    impl = GodunovImplemGB300(MHDSettings(gamma0=1.4, cfl=0.4, slope_type=2.0, riemann="HLLD", viscosity_mu=mu or None,
+                                          gravity=gravity), mesh, precision="mixed")
     U, B = (torch.from_numpy(a).cuda() for a in _state(mesh))
     U2, B2 = torch.zeros_like(U), torch.zeros_like(B)
-    impl.do_time_step(U, U2, B, B2, 2.0 ** -13)
+    impl.do_time_step(U, U2, B, B2, dt)
     n = mesh.n_owned
     out = hashlib.sha256(U2[:n].cpu().numpy().tobytes() + B2[:n].cpu().numpy().tobytes()).hexdigest()[:16]
     impl.close()
@@ -97,3 +97,36 @@ DIGESTS = {
 @pytest.mark.parametrize("mu", [0.0, 1e-3])
 def test_step_rounds_as_recorded(dim, block, amr, mu):
     assert digest(dim, block, amr, mu) == DIGESTS[dim, block, amr, mu]
+
+
+# strong gravity along every axis, a time step that is no power of two (with one, the kick's product is exact)
+GRAVITY = dict(gravity=(40.0, -70.0, 55.0), dt=1.1371 * 2.0 ** -13)
+DIGESTS_GRAVITY = {
+    (2, 16, False, 0.0): "464faf66387fafe9",
+    (2, 16, False, 0.001): "355e386b6b450ab5",
+    (2, 16, True, 0.0): "7b849d38a8255a06",
+    (2, 16, True, 0.001): "079effc793a5bd62",
+    (2, 8, False, 0.0): "72e6feceb810ea53",
+    (2, 8, False, 0.001): "b22418929c599d21",
+    (2, 8, True, 0.0): "007f86afb3612fb7",
+    (2, 8, True, 0.001): "206cc47310802d64",
+    (2, 12, False, 0.0): "7d1e60551e9d7839",
+    (2, 12, False, 0.001): "22bfba4ceaf106b1",
+    (2, 12, True, 0.0): "7ea97a9095eab997",
+    (2, 12, True, 0.001): "3b050312b9a4573e",
+    (3, 16, False, 0.0): "b865db712fa14198",
+    (3, 16, False, 0.001): "5d408451215c48a7",
+    (3, 16, True, 0.0): "e4a137b032fbf704",
+    (3, 16, True, 0.001): "e5dcca840486961f",
+    (3, 12, False, 0.0): "c4a6917d8e3265f5",
+    (3, 12, False, 0.001): "d30e02fa96c80de9",
+    (3, 12, True, 0.0): "b722a3a2d1896a62",
+    (3, 12, True, 0.001): "21b85d9c20e8c848",
+}
+
+
+@pytest.mark.parametrize("dim,block", [(2, 16), (2, 8), (2, 12), (3, 16), (3, 12)])
+@pytest.mark.parametrize("amr", [False, True])
+@pytest.mark.parametrize("mu", [0.0, 1e-3])
+def test_step_with_gravity_rounds_as_recorded(dim, block, amr, mu):
+    assert digest(dim, block, amr, mu, **GRAVITY) == DIGESTS_GRAVITY[dim, block, amr, mu]
