@@ -24,9 +24,10 @@ namespace gmhd
 
 // Programmatic dependent launch (gmhd_advance): a kernel lets the next one of its stream start as soon as all of its own
 // CTAs have, and reads nothing that a kernel before may write until that one has ended. The launch latency and the
-// first instructions of the next kernel then run beside the last wave of this one. 2D 128^2, mixed: 25.7 us a step with
-// full dependences and a clearing of the CFL maxima between two kernels, 21.1 us now. (Setting the time step in the
-// step's last CTA instead: 24.2 us, and its fence and ticket at the end of each CTA cost meshes of many tiles 6 %.)
+// first instructions of the next kernel then run beside the last wave of this one. 2D 128^2, mixed, in 16x16 tiles: 25.7 us a
+// step with full dependences and a clearing of the CFL maxima between two kernels, 21.1 us like this (17.6 in the 8x8 tiles that
+// such a mesh takes now). (Setting the time step in the step's last CTA instead: 24.2 us, and its fence and ticket at the
+// end of each CTA cost meshes of many tiles 6 %.)
 __device__ __forceinline__ void
 next_kernel_may_start()
 {

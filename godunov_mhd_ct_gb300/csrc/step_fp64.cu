@@ -100,8 +100,11 @@ tile_shape_fp64(int dim, int bx, int by, int bz, bool visc, int tile, int * t)
 int
 default_tile_fp64(int dim, int bx, int by, int bz, int n_owned)
 {
-  // (FP64 results do not depend on the tile.) 2D: 64 tiles of 16x16 took 154 us, as 8x8 tiles 94 us; 128 tiles 153
-  // against 174. 3D: 32 tiles of 8x4x4 took 175 us, as 4x4x4 tiles 119 us; 96 tiles 174 against 222.
+  // (FP64 results do not depend on the tile.) Largest against small tiles, us a step. Uniform, small ones _W: 2D, 64 tiles of
+  // 16x16 138 / 81, 80 138 / 130; 3D, 64 tiles of 8x4x4 146 / 107, 96 145 / 175. Without a _W variant the small tiles gain less.
+  // Coarse/fine: 2D, 22 to 76 tiles 295 / 250, with viscosity 320 / 266 (88 298 / 261, 323 / 276: the line could lie
+  // higher there); 3D, 60 tiles 325 / 319, with viscosity 367 / 358, 116 tiles 326 / 356, 367 / 397. Uniform with viscosity:
+  // 2D, 1 to 64 tiles 147 / 120, 80 146 / 135; 3D, 64 tiles 161 / 158, 96 161 / 190.
   const long long half = kSMs / 2;
   if (dim == 2 && bx % 16 == 0 && by % 16 == 0 && (long long)n_owned * (bx / 16) * (by / 16) <= half)
     return 8;

@@ -34,7 +34,8 @@ tiles_of(const StepArgs & a, int dim, int n)
 }
 
 // Meshes of at most half as many of their largest tiles as SMs, when no tile was asked for, run as smaller ones: the same
-// results on more SMs. Twenty steps, us: 2D, 1 / 64 / 81 tiles of 16x16 421 / 437 / 590, as 8x8 with 256 threads 350 / 378 /
+// results on more SMs. (Viscous meshes do not: 64 tiles of 16x16 take 14.7 us a step, as 8x8 16.6; 16 tiles of 8x8x4 24.9, as
+// 4x4x4 29.0.) Twenty steps, us: 2D, 1 / 64 / 81 tiles of 16x16 421 / 437 / 590, as 8x8 with 256 threads 350 / 378 /
 // 678. 3D, 8 / 64 / 125 tiles of 8x8x8 863 / 858 / 1395, as 4x4x4 with 96 threads 717 / 769 / 1887 (with 256: 489 for 8).
 static bool
 few_tiles(const StepArgs & a, int dim)
