@@ -500,20 +500,23 @@ namespace gmhd
 
 // Both kernels are bound by the FP64 pipe (two lanes an SM): divisions, maxima and halvings are integer sequences with the
 // same results, and the indicator's quotients are compared in FP32 before one of a warp is formed. 2D, 3.5 k blocks of
-// 16^2, rho and the pressure: 155 + 133 us before, 43 + 47 us now.
+// 16^2, rho and the pressure: 155 + 133 us before, 43 + 47 us now. Blocks of 4^2 are bound by their CTAs and idle lanes: 65 k of
+// them, the whole call 714 us before, 962 with a CTA of the first kernel for each, 455 now.
 
 // quantity 0 (rho) or 1 (pressure) of every owned cell, into q[var][block][cell]; a CTA takes 256 cells of a block at a time
+// (`chunks` of them a block), or `per` whole blocks of fewer cells: with one block of 4^2 a CTA 15 of 16 threads had none
 __global__ void __launch_bounds__(256)
-refine_quantity_kernel(const double * __restrict__ U, const double * __restrict__ B, int n_owned, int chunks, int dim,
-                       int bx, int by, int64_t ncell, int64_t nfx, int64_t nfy, int64_t nface, double gamma0,
+refine_quantity_kernel(const double * __restrict__ U, const double * __restrict__ B, int n_owned, int chunks, int per,
+                       int dim, int bx, int by, int64_t ncell, int64_t nfx, int64_t nfy, int64_t nface, double gamma0,
                        double smallr, double smallp, int use_rho, int use_pressure, double * __restrict__ q)
 {
-  const int64_t total = (int64_t)n_owned * ncell, n_work = (int64_t)n_owned * chunks;
+  const int64_t total = (int64_t)n_owned * ncell, n_work = (int64_t)((n_owned + per - 1) / per) * chunks;
+  const int     tid = (int)threadIdx.x, sub = per > 1 ? tid / (int)ncell : 0;
   for (int64_t w = blockIdx.x; w < n_work; w += gridDim.x)
   {
-    const int64_t blk = w / chunks;
-    const int     c = (int)(w - blk * chunks) * 256 + (int)threadIdx.x;
-    if (c >= ncell)
+    const int64_t blk = per > 1 ? w * per + sub : w / chunks;
+    const int     c = per > 1 ? tid - sub * (int)ncell : (int)(w - blk * chunks) * 256 + tid;
+    if (sub >= per || blk >= n_owned || c >= ncell)
       continue;
     const double *Ub = U + blk * 5 * ncell, *Bb = B + blk * nface;
     const int64_t g = blk * ncell + c;
@@ -581,6 +584,8 @@ refine_flags_kernel(const double * __restrict__ q, int nvar, const int32_t * __r
     const double * Q = q + ((int64_t)var * n_owned + blk) * ncell;
     for (int c0 = 0; c0 < ncell; c0 += 256)
     {
+      if (c0 + (int)(threadIdx.x & ~31u) >= ncell)
+        break; // a warp without a cell
       const int    c = c0 + (int)threadIdx.x;
       const bool   in = c < ncell;
       const int    i = c % bx, jk = c / bx, j = jk % by, k = jk / by;
@@ -632,10 +637,10 @@ launch_refine_flags(const double * U, const double * B, const int32_t * level, i
 {
   if (n_owned <= 0)
     return 0;
-  const int     chunks = (int)((ncell + 255) / 256);
-  const int64_t want = (int64_t)n_owned * chunks;
+  const int     chunks = (int)((ncell + 255) / 256), per = ncell < 256 ? 256 / (int)ncell : 1;
+  const int64_t want = (int64_t)((n_owned + per - 1) / per) * chunks;
   refine_quantity_kernel<<<(int)(want < kSMs * 64 ? want : kSMs * 64), 256, 0, stream>>>(
-    U, B, n_owned, chunks, dim, bx, by, ncell, nfx, nfy, nface, gamma0, smallr, smallp, use_rho, use_pressure, scratch);
+    U, B, n_owned, chunks, per, dim, bx, by, ncell, nfx, nfy, nface, gamma0, smallr, smallp, use_rho, use_pressure, scratch);
   refine_flags_kernel<<<n_owned, 256, 0, stream>>>(scratch, (use_rho ? 1 : 0) + (use_pressure ? 1 : 0), level, n_owned,
                                                    dim, bx, by, bz, ncell, criterion, level_min, level_max, eps_refine,
                                                    eps_coarsen, eps_lohner, flags);
